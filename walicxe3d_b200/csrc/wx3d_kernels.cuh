@@ -63,12 +63,12 @@ struct Geo {
 };
 
 // Ring channels per cell: the primitives, plus -- for the first-order hydro
-// stage, whose interface states are the cell values -- the sound speed and
-// 1/rho, computed once when the plane is loaded instead of at each of the
-// six interfaces that use the cell.
+// stage, whose interface states are the cell values -- the sound speed,
+// computed once when the plane is loaded instead of at each of the six
+// interfaces that use the cell.
 template <int NEQ, bool MHD, int ORDER>
 __host__ __device__ constexpr int ring_channels() {
-  return NEQ + ((!MHD && ORDER == 1) ? 2 : 0);
+  return NEQ + ((!MHD && ORDER == 1) ? 1 : 0);
 }
 
 constexpr int VPLANE = (NC + 2) * (NC + 2);  // a plane with its one-deep x/y frame
@@ -161,25 +161,21 @@ __device__ __forceinline__ void iface_flux(const double* c0, const double* c1, c
       pr[e] = pr[e] - 0.5 * ar;
     }
   }
-  if constexpr (!MHD && (SOLVER == WX_SOLVER_HLL || SOLVER == WX_SOLVER_HLLC)) {
-    double cl, cr, rl, rr;
-    if constexpr (ORDER == 1) {  // cell values: sound speed and 1/rho from the ring
+  if constexpr (!MHD) {
+    double cl, cr;
+    if constexpr (ORDER == 1) {  // cell values: sound speed from the ring
       cl = c1[NEQ * Geo<ORDER>::PL];
       cr = c2[NEQ * Geo<ORDER>::PL];
-      rl = c1[(NEQ + 1) * Geo<ORDER>::PL];
-      rr = c2[(NEQ + 1) * Geo<ORDER>::PL];
     } else {
-      rl = rcp_nr(pl[0]);
-      rr = rcp_nr(pr[0]);
-      cl = sqrt_nr(ph.gamma * pl[4] * rl);
-      cr = sqrt_nr(ph.gamma * pr[4] * rr);
+      cl = sound_nr(ph.gamma * pl[4], pl[0]);
+      cr = sound_nr(ph.gamma * pr[4], pr[0]);
     }
-    if constexpr (SOLVER == WX_SOLVER_HLLC) riemann_hllc_c<NEQ>(pl, pr, cl, cr, rl, rr, fx, ph.cv);
+    if constexpr (SOLVER == WX_SOLVER_HLLC) riemann_hllc_c<NEQ>(pl, pr, cl, cr, fx, ph.cv);
     else riemann_hll_c<NEQ>(pl, pr, cl, cr, fx, ph.cv);
   } else {
 #pragma unroll
     for (int e = 0; e < NEQ; ++e) fx[e] = 0.0;
-    riemann<NEQ, MHD, SOLVER>(pl, pr, fx, ph.gamma, ph.cv);
+    riemann_mhd<NEQ, SOLVER>(pl, pr, fx, ph.gamma, ph.cv);
   }
 #pragma unroll
   for (int e = 0; e < NEQ; ++e) f[perm<DIR, MHD>(e)] = fx[e];
@@ -208,7 +204,7 @@ __device__ __forceinline__ void visc_store(const StageParams& P, const DevBlock&
 // physical cells, plus -- for the planes that get x/y fluxes -- the x/y ghost
 // frame (two deep for the second-order stage), gathered from the neighbours.
 // Converts one cell's conserved variables to primitives (plus, for the
-// first-order hydro stage, its sound speed and 1/rho) into ring plane pl,
+// first-order hydro stage, its sound speed) into ring plane pl,
 // counting the flow2prim floors of physical cells when `count`.
 template <int NEQ, bool MHD, int ORDER, int CH>
 __device__ __forceinline__ void store_cell(const PhysParams& ph, double* pl, int i, int j, const double* u, bool count,
@@ -217,7 +213,6 @@ __device__ __forceinline__ void store_cell(const PhysParams& ph, double* pl, int
   const int st = flow2prim<NEQ, MHD>(u, p, ph.inv_cv, &rinv);
   if constexpr (CH > NEQ) {
     pl[NEQ * Geo<ORDER>::PL + hidx<ORDER>(i, j)] = sqrt_nr(ph.gamma * p[4] * rinv);
-    pl[(NEQ + 1) * Geo<ORDER>::PL + hidx<ORDER>(i, j)] = rinv;
   }
   if (count && st != 0) atomicAdd(&cnt[st == 1 ? 0 : (st == 2 ? 1 : 2)], 1u);
 #pragma unroll
