@@ -50,7 +50,13 @@ struct Kern {
 template <int NEQ, bool MHD, int SOLVER, int LIM>
 Kern make_kern() {
   Kern k;
-  k.stage1 = stage_kernel<NEQ, MHD, SOLVER, 1, LIM_RUNTIME>;
+  if constexpr (MHD) {
+    k.stage1 = stage_kernel<NEQ, true, SOLVER, 1, LIM_RUNTIME>;
+    k.smem1 = stage_smem_bytes<NEQ, true, 1>();
+  } else {
+    k.stage1 = predictor_kernel<NEQ, SOLVER>;
+    k.smem1 = sizeof(PredSmem<NEQ>);
+  }
   k.stage2 = stage_kernel<NEQ, MHD, SOLVER, 2, LIM>;
   k.stage2v = stage_kernel<NEQ, MHD, SOLVER, 2, LIM, true>;
   k.lax = lax_kernel<NEQ, MHD>;
@@ -60,7 +66,6 @@ Kern make_kern() {
   k.src = source_kernel<NEQ, MHD>;
   k.mark = mark_kernel<NEQ, MHD>;
   k.prims = prims_kernel<NEQ, MHD>;
-  k.smem1 = stage_smem_bytes<NEQ, MHD, 1>();
   k.smem2 = stage_smem_bytes<NEQ, MHD, 2>();
   k.smem2v = stage_smem_bytes<NEQ, MHD, 2, true>();
   return k;

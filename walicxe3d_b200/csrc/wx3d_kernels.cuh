@@ -530,6 +530,270 @@ __global__ void __launch_bounds__(STAGE_THREADS, (stage_ctas_per_sm<NEQ, MHD, OR
 }
 
 // ---------------------------------------------------------------------------
+// First-order stage of the hydro equations (the predictor, and the single
+// stage of HLL1): one CTA per (block, z-slab), marching up the z-planes.
+//
+// What bounds the stage is the shared-memory/L1 data path (67 % busy in the
+// stage kernel that staged every operand and every flux through shared
+// memory), then instruction issue, so as little as possible travels:
+//  - a thread t < 256 owns a column and keeps the primitives (and sound
+//    speed) of its cell of plane m in registers for its three interfaces;
+//  - it solves the x-interface to the next cell and the y-interface to the
+//    next row, reading only that neighbour's primitives from the plane in
+//    shared memory; the x-flux goes to the next lane by a shuffle, the
+//    y-flux to the next row through shared memory;
+//  - the frame cells never reach shared memory: each of the 64 threads of
+//    warps 8 and 9 gathers the ghost of one (side, row), keeps it in
+//    registers and solves the block-face interface it belongs to (x on
+//    warp 8, y on warp 9), so no warp has a partly filled solve.
+// The plane and the flux buffers are doubled, which leaves one barrier per
+// plane: the update of plane m and the fluxes of plane m+1 run between the
+// same two barriers.  Conserved cells arrive by 8-byte asynchronous copies a
+// plane ahead and stay in shared memory until they are the base of the
+// update (P.base is P.src), so no load holds registers across the fluxes:
+// with 96 registers and no spills two CTAs share an SM.  Loading them into
+// registers instead, or late, spilled or exposed the loads (1.71 and 1.95 ms
+// against 1.51 on the 11,600-block AMR blast at five equations; the kernel
+// that staged everything took 1.75); three CTAs at 64 registers: 2.06 ms.
+// Six equations, 5,496 blocks of the winds mesh: 0.945 -> 0.848 ms.
+template <int NEQ>
+struct PredSmem {
+  static constexpr int W = NC + 1;               // padded row: a column read is conflict-free
+  double pl[2][NEQ + 1][W * NC];                 // primitives and sound speed of a plane
+  double raw[3][NEQ][PLANE];                     // conserved variables of planes m, m+1, m+2
+  double fy[2][NEQ][(NC + 1) * NC];              // y-flux below row j (rows 0 and 16: block faces)
+  double ex[2][2][NEQ][NC];                      // x-flux of the low and the high block face
+  DevBlock B;
+  StageConsts K;
+};
+
+// Barrier of all threads of a stage CTA, met by the roles at different places.
+__device__ __forceinline__ void plane_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(STAGE_THREADS) : "memory"); }
+__device__ __forceinline__ void copy_async8(double* smem, const double* g) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(g) : "memory");
+}
+__device__ __forceinline__ void copy_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+template <int NEQ, int SOLVER, int DIR>
+__device__ __forceinline__ void cell_flux(const double* a, const double* b, const PhysParams& ph, double* f) {
+  double pl[NEQ], pr[NEQ], fx[NEQ];
+#pragma unroll
+  for (int e = 0; e < NEQ; ++e) {
+    pl[e] = a[perm<DIR, false>(e)];
+    pr[e] = b[perm<DIR, false>(e)];
+  }
+  if constexpr (SOLVER == WX_SOLVER_HLLC) riemann_hllc_c<NEQ>(pl, pr, a[NEQ], b[NEQ], fx, ph.cv);
+  else riemann_hll_c<NEQ>(pl, pr, a[NEQ], b[NEQ], fx, ph.cv);
+#pragma unroll
+  for (int e = 0; e < NEQ; ++e) f[perm<DIR, false>(e)] = fx[e];
+}
+
+// Primitives and sound speed of a cell; physical cells count their floors.
+template <int NEQ>
+__device__ __forceinline__ void prim_and_sound(const PhysParams& ph, const double* u, double* p, bool count,
+                                               unsigned* cnt) {
+  double rinv;
+  const int st = flow2prim<NEQ, false>(u, p, ph.inv_cv, &rinv);
+  p[NEQ] = sqrt_nr(ph.gamma * p[4] * rinv);
+  if (count && st != 0) atomicAdd(&cnt[st == 1 ? 0 : (st == 2 ? 1 : 2)], 1u);
+}
+
+template <int NEQ, int SOLVER>
+__global__ void __launch_bounds__(STAGE_THREADS, 2) predictor_kernel(StageParams P) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  PredSmem<NEQ>& S = *reinterpret_cast<PredSmem<NEQ>*>(smraw);
+  constexpr int W = PredSmem<NEQ>::W;
+  DevBlock& B = S.B;
+  StageConsts& K = S.K;
+  const int t = threadIdx.x, lane = t & (NC - 1);
+  const PhysParams& ph = P.ph;
+  const int planes = NC / P.zsplit;
+  const bool column = t < PLANE;
+  const int ci = lane + 1, cj = (t >> 4) + 1;                  // column threads
+  const int side = (t - PLANE) >> 4;                           // face threads: 0, 1 x; 2, 3 y
+  const int gi = side == 0 ? 0 : (side == 1 ? NC + 1 : lane + 1);
+  const int gj = side == 2 ? 0 : (side == 3 ? NC + 1 : lane + 1);
+  const double* gsrc = P.gsrc ? P.gsrc : P.src;
+  if (t < 4) K.cnt[t] = 0;
+
+  for (int w = blockIdx.x; w < P.nwork;) {
+    const int slot = P.work[w / P.zsplit];
+    const int z0 = 1 + (w % P.zsplit) * planes, z1 = z0 + planes - 1;
+    __syncthreads();
+    if (t < (int)(sizeof(DevBlock) / 4)) reinterpret_cast<int*>(&B)[t] = reinterpret_cast<const int*>(P.blocks + slot)[t];
+    __syncthreads();
+    if (t == 0) {  // read after the prologue's barrier
+      const double dtp = P.ctl->dt * P.dt_factor;
+      K.dtdx = dtp / B.dx;
+      K.dtdy = dtp / B.dy;
+      K.dtdz = dtp / B.dz;
+    }
+    // conserved variables of the column's cell of plane kk into the raw ring
+    // (an asynchronous copy; each thread reads back its own cell only)
+    auto fetch = [&](int kk) {
+      double* d = &S.raw[(unsigned)(kk + 3) % 3u][0][t];
+      if (kk >= 1 && kk <= NC) {
+        const double* g = P.src + cell_off(slot, NEQ, 0, ci, cj, kk);
+#pragma unroll
+        for (int e = 0; e < NEQ; ++e) copy_async8(d + e * PLANE, g + (size_t)e * BCELLS);
+      } else {
+        double u[NEQ];
+        gather_ghost<NEQ>(gsrc, B, slot, ci, cj, kk, u);
+#pragma unroll
+        for (int e = 0; e < NEQ; ++e) d[e * PLANE] = u[e];
+      }
+    };
+    // primitives and sound speed of the column's cell of plane kk
+    auto convert = [&](int kk, double* p) {
+      const double* d = &S.raw[(unsigned)(kk + 3) % 3u][0][t];
+      double u[NEQ];
+#pragma unroll
+      for (int e = 0; e < NEQ; ++e) u[e] = d[e * PLANE];
+      prim_and_sound<NEQ>(ph, u, p, kk >= z0 && kk <= z1, K.cnt);
+    };
+    auto put_plane = [&](int kk, const double* p) {
+      double* d = &S.pl[kk & 1][0][(cj - 1) * W + lane];
+#pragma unroll
+      for (int e = 0; e <= NEQ; ++e) d[e * (W * NC)] = p[e];
+    };
+    auto put_mark = [&](int e, const double* p) {  // (rho, p) of a ghost cell for markByPhysical
+      double2 v;
+      v.x = p[0];
+      v.y = p[4];
+      reinterpret_cast<double2*>(P.gframe)[(size_t)slot * GFRAME + e] = v;
+    };
+    double pc[NEQ + 1], zf[NEQ];
+    if (column) {
+      double pn[NEQ + 1];
+      fetch(z0 - 1);
+      fetch(z0);
+      fetch(z0 + 1);
+      copy_async_wait();
+      convert(z0 - 1, pn);
+      if (P.gframe && z0 == 1) put_mark(gframe_entry(0, t), pn);
+      if (z0 + 2 <= z1 + 1) fetch(z0 + 2);   // into the slot of plane z0-1
+      convert(z0, pc);
+      put_plane(z0, pc);
+      cell_flux<NEQ, SOLVER, 2>(pn, pc, ph, zf);
+      convert(z0 + 1, pn);
+      if (P.gframe && z0 + 1 == NC + 1) put_mark(gframe_entry(NC + 1, t), pn);
+      put_plane(z0 + 1, pn);
+    } else {
+      double u[NEQ];
+      gather_ghost<NEQ>(gsrc, B, slot, gi, gj, z0, u);
+      prim_and_sound<NEQ>(ph, u, pc, false, K.cnt);
+      if (P.gframe) put_mark(gframe_entry(z0, t), pc);
+    }
+    __syncthreads();
+
+    for (int m = z0; m <= z1; ++m) {
+      const int b = m & 1;
+      if (column) {
+        double dx[NEQ], dz[NEQ], f[NEQ];
+        const double* pl = &S.pl[b][0][(cj - 1) * W + lane];
+        {  // y-interface to row cj+1 (the last row's flux is a face thread's)
+          double pr[NEQ + 1];
+          const int o = cj < NC ? W : 0;
+#pragma unroll
+          for (int e = 0; e <= NEQ; ++e) pr[e] = pl[e * (W * NC) + o];
+          cell_flux<NEQ, SOLVER, 1>(pc, pr, ph, f);
+          if (cj < NC) {
+#pragma unroll
+            for (int e = 0; e < NEQ; ++e) S.fy[b][e][cj * NC + lane] = f[e];
+          }
+        }
+        {  // x-interface to cell ci+1 (the last lane's flux is a face thread's)
+          double pr[NEQ + 1];
+          const int o = lane < NC - 1 ? 1 : 0;
+#pragma unroll
+          for (int e = 0; e <= NEQ; ++e) pr[e] = pl[e * (W * NC) + o];
+          cell_flux<NEQ, SOLVER, 0>(pc, pr, ph, f);
+#pragma unroll
+          for (int e = 0; e < NEQ; ++e) {
+            const double xl = __shfl_up_sync(0xffffffffu, f[e], 1, NC);
+            dx[e] = lane == 0 ? -f[e] : (lane == NC - 1 ? xl : xl - f[e]);
+          }
+        }
+        {  // z-interface m+1/2: the column's own cells
+          const double* pu = &S.pl[b ^ 1][0][(cj - 1) * W + lane];
+          double pn[NEQ + 1];
+#pragma unroll
+          for (int e = 0; e <= NEQ; ++e) pn[e] = pu[e * (W * NC)];
+          cell_flux<NEQ, SOLVER, 2>(pc, pn, ph, f);
+#pragma unroll
+          for (int e = 0; e < NEQ; ++e) {
+            dz[e] = zf[e] - f[e];
+            zf[e] = f[e];
+          }
+#pragma unroll
+          for (int e = 0; e <= NEQ; ++e) pc[e] = pn[e];
+        }
+        const size_t o = cell_off(slot, NEQ, 0, ci, cj, m);
+        plane_barrier();
+        // conservative update of plane m (godunov.f90:259-271); each
+        // direction's two fluxes are subtracted before they are scaled, so
+        // equal fluxes cancel exactly
+        const double dtdx = K.dtdx, dtdy = K.dtdy, dtdz = K.dtdz;
+        const bool xedge = lane == 0 || lane == NC - 1;
+        const double* ex = &S.ex[b][lane >> 3][0][cj - 1];
+        const double* v = &S.raw[(unsigned)m % 3u][0][t];
+#pragma unroll
+        for (int e = 0; e < NEQ; ++e) {
+          const double xe = xedge ? ex[e * NC] : 0.0;
+          const double ddx = dx[e] + (lane == 0 ? xe : -xe);
+          const double dy = S.fy[b][e][(cj - 1) * NC + lane] - S.fy[b][e][cj * NC + lane];
+          P.out[o + (size_t)e * BCELLS] = v[e * PLANE] + dtdx * ddx + dtdy * dy + dtdz * dz[e];
+        }
+        if (m < z1) {  // plane m+2 into the buffer of plane m, which no one reads any more
+          double pn[NEQ + 1];
+          copy_async_wait();
+          convert(m + 2, pn);
+          if (P.gframe && m + 2 == NC + 1) put_mark(gframe_entry(NC + 1, t), pn);
+          put_plane(m + 2, pn);
+          if (m + 3 <= z1 + 1) fetch(m + 3);
+        }
+      } else {
+        double u[NEQ], pr[NEQ + 1], f[NEQ];
+        if (m < z1) gather_ghost<NEQ>(gsrc, B, slot, gi, gj, m + 1, u);
+        if (side < 2) {
+          const double* c = &S.pl[b][0][lane * W + (side ? NC - 1 : 0)];
+#pragma unroll
+          for (int e = 0; e <= NEQ; ++e) pr[e] = c[e * (W * NC)];
+          double l[NEQ + 1], r[NEQ + 1];
+#pragma unroll
+          for (int e = 0; e <= NEQ; ++e) { l[e] = side ? pr[e] : pc[e]; r[e] = side ? pc[e] : pr[e]; }
+          cell_flux<NEQ, SOLVER, 0>(l, r, ph, f);
+#pragma unroll
+          for (int e = 0; e < NEQ; ++e) S.ex[b][side][e][lane] = f[e];
+        } else {
+          const double* c = &S.pl[b][0][(side == 3 ? NC - 1 : 0) * W + lane];
+#pragma unroll
+          for (int e = 0; e <= NEQ; ++e) pr[e] = c[e * (W * NC)];
+          double l[NEQ + 1], r[NEQ + 1];
+#pragma unroll
+          for (int e = 0; e <= NEQ; ++e) { l[e] = side == 3 ? pr[e] : pc[e]; r[e] = side == 3 ? pc[e] : pr[e]; }
+          cell_flux<NEQ, SOLVER, 1>(l, r, ph, f);
+#pragma unroll
+          for (int e = 0; e < NEQ; ++e) S.fy[b][e][(side == 3 ? NC * NC : 0) + lane] = f[e];
+        }
+        plane_barrier();
+        if (m < z1) {
+          prim_and_sound<NEQ>(ph, u, pc, false, K.cnt);
+          if (P.gframe) put_mark(gframe_entry(m + 1, t), pc);
+        }
+      }
+    }
+    // items past the first wave go, in list order, to whichever CTA
+    // finishes first (the counter is zeroed before each launch)
+    if (t == 0) K.next = (int)gridDim.x + (int)atomicAdd(&P.ctl->work_next[0], 1u);
+    __syncthreads();
+    w = K.next;
+  }
+  __syncthreads();
+  if (t < 4 && K.cnt[t]) atomicAdd(&P.ctl->cnt[t], (unsigned long long)K.cnt[t]);
+}
+
+// ---------------------------------------------------------------------------
 // Lax-Friedrichs (lax.f90:39-99): first order, from U with one-deep ghosts.
 struct LaxParams {
   const double* __restrict__ u;
