@@ -51,14 +51,20 @@ template <int NEQ, bool MHD, int SOLVER, int LIM>
 Kern make_kern() {
   Kern k;
   if constexpr (MHD) {
-    k.stage1 = stage_kernel<NEQ, true, SOLVER, 1, LIM_RUNTIME>;
-    k.smem1 = stage_smem_bytes<NEQ, true, 1>();
+    k.stage1 = stage_kernel<NEQ, SOLVER, 1, LIM_RUNTIME>;
+    k.stage2 = stage_kernel<NEQ, SOLVER, 2, LIM>;
+    k.stage2v = stage_kernel<NEQ, SOLVER, 2, LIM, true>;
+    k.smem1 = stage_smem_bytes<NEQ, 1>();
+    k.smem2 = stage_smem_bytes<NEQ, 2>();
+    k.smem2v = stage_smem_bytes<NEQ, 2, true>();
   } else {
     k.stage1 = predictor_kernel<NEQ, SOLVER>;
+    k.stage2 = corrector_kernel<NEQ, SOLVER, LIM, false>;
+    k.stage2v = corrector_kernel<NEQ, SOLVER, LIM, true>;
     k.smem1 = sizeof(PredSmem<NEQ>);
+    k.smem2 = sizeof(CorrSmem<NEQ, false>);
+    k.smem2v = sizeof(CorrSmem<NEQ, true>);
   }
-  k.stage2 = stage_kernel<NEQ, MHD, SOLVER, 2, LIM>;
-  k.stage2v = stage_kernel<NEQ, MHD, SOLVER, 2, LIM, true>;
   k.lax = lax_kernel<NEQ, MHD>;
   k.visc = viscous_kernel<NEQ, MHD>;
   k.dt = dt_kernel<NEQ, MHD>;
@@ -66,8 +72,6 @@ Kern make_kern() {
   k.src = source_kernel<NEQ, MHD>;
   k.mark = mark_kernel<NEQ, MHD>;
   k.prims = prims_kernel<NEQ, MHD>;
-  k.smem2 = stage_smem_bytes<NEQ, MHD, 2>();
-  k.smem2v = stage_smem_bytes<NEQ, MHD, 2, true>();
   return k;
 }
 

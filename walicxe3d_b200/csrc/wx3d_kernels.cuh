@@ -1,9 +1,13 @@
 // wx3d_kernels.cuh -- sm_100a kernels of the per-block Godunov update.
 //
-// Stage kernel: one CTA per (block, z-slab).  320 threads (10 warps) march
-// through the slab's k-planes; a 4-plane shared-memory ring holds the
-// primitives of each plane together with its two-deep x/y ghost frame, so
-// every x-, y- and z-interface flux is computed exactly once and the
+// Stages of the Godunov step, one CTA per (block, z-slab) marching up the
+// slab's k-planes: predictor_kernel and corrector_kernel for the hydro
+// equations, stage_kernel (either order) for MHD.  All are persistent: items
+// past the first wave are handed out on demand.
+//
+// stage_kernel: 320 threads (10 warps); a 4-plane shared-memory ring holds
+// the primitives of each plane together with its ORDER-deep x/y ghost frame,
+// so every x-, y- and z-interface flux is computed exactly once and the
 // conservative update (godunov.f90:259-271) reads the two fluxes of each
 // face from shared memory (x, y) or from the thread's registers (z).
 #pragma once
@@ -14,9 +18,10 @@
 namespace wx {
 
 
-// 17*16 x- and y-interfaces per plane on the first 272 threads; the plane
-// loads (320 cells at first order, 384 at second) spread over all 320, and
-// two CTAs per SM put five warps on every sub-partition
+// stage_kernel: 17*16 x- and y-interfaces per plane on the first 272 threads,
+// the plane loads (320 cells at first order, 384 at second) over all 320.
+// predictor_kernel, corrector_kernel: 256 columns and 64 block-face cells of
+// a plane; two CTAs per SM put five warps on every sub-partition.
 constexpr int STAGE_THREADS = 320;
 static_assert(STAGE_THREADS >= 17 * NC, "one thread per x- and y-interface of a plane");
 static_assert(STAGE_THREADS >= PLANE + 4 * NC, "the viscous step's UP frame is gathered by threads PLANE..PLANE+63");
@@ -24,7 +29,7 @@ constexpr int RING = 4;             // planes p-1..p+2 of the second-order stenc
 
 struct StageParams {
   const double* __restrict__ src;   // array whose primitives feed the fluxes (physical cells)
-  const double* __restrict__ base;  // array the update starts from (U)
+  const double* __restrict__ base;  // array the update starts from (U; src itself at first order)
   double* __restrict__ out;         // result (UP for stage 1, W for stage 2)
   const DevBlock* __restrict__ blocks;
   const int32_t* __restrict__ work; // occupied slots
@@ -62,15 +67,6 @@ struct Geo {
   static constexpr int PL = W * W;
 };
 
-// Ring channels per cell: the primitives, plus -- for the first-order hydro
-// stage, whose interface states are the cell values -- the sound speed,
-// computed once when the plane is loaded instead of at each of the six
-// interfaces that use the cell.
-template <int NEQ, bool MHD, int ORDER>
-__host__ __device__ constexpr int ring_channels() {
-  return NEQ + ((!MHD && ORDER == 1) ? 1 : 0);
-}
-
 constexpr int VPLANE = (NC + 2) * (NC + 2);  // a plane with its one-deep x/y frame
 
 // Per-block constants and status counters of a stage CTA, kept in shared
@@ -84,9 +80,9 @@ struct StageConsts {
   int pad_;
 };
 
-template <int NEQ, bool MHD, int ORDER, bool VISC = false>
+template <int NEQ, int ORDER, bool VISC = false>
 __host__ __device__ constexpr size_t stage_smem_bytes() {
-  return sizeof(double) * ((size_t)RING * ring_channels<NEQ, MHD, ORDER>() * Geo<ORDER>::PL + 2 * (size_t)NEQ * 17 * NC +
+  return sizeof(double) * ((size_t)RING * NEQ * Geo<ORDER>::PL + 2 * (size_t)NEQ * 17 * NC +
                            (VISC ? 2 * (size_t)NEQ * VPLANE : 0)) +
          sizeof(DevBlock) + sizeof(StageConsts);
 }
@@ -135,21 +131,21 @@ __device__ __forceinline__ void flush_counts(DevCtl* ctl, unsigned pf, unsigned 
 // the previous interface -- the limiter sees the same two differences -- and
 // is taken from `carry` instead of being evaluated again, unless `first`;
 // the upper cell's slope is left in `carry` for the next interface.
-template <int NEQ, bool MHD, int SOLVER, int ORDER, int LIM, int DIR, bool CARRY = false>
+template <int NEQ, int SOLVER, int ORDER, int LIM, int DIR, bool CARRY = false>
 __device__ __forceinline__ void iface_flux(const double* c0, const double* c1, const double* c2, const double* c3,
                                            const PhysParams& ph, double* f, double* carry = nullptr,
                                            bool first = true) {
   double pl[NEQ], pr[NEQ], fx[NEQ];
 #pragma unroll
   for (int e = 0; e < NEQ; ++e) {
-    const int q = perm<DIR, MHD>(e);
+    const int q = perm<DIR, true>(e);
     pl[e] = c1[q * Geo<ORDER>::PL];
     pr[e] = c2[q * Geo<ORDER>::PL];
   }
   if (ORDER == 2) {  // limiter (hydro_core.f90:613-636) on permuted primitives
 #pragma unroll
     for (int e = 0; e < NEQ; ++e) {
-      const int q = perm<DIR, MHD>(e);
+      const int q = perm<DIR, true>(e);
       const double prr = c3[q * Geo<ORDER>::PL];
       const double dm = pr[e] - pl[e], dr = prr - pr[e];
       double al;
@@ -161,24 +157,11 @@ __device__ __forceinline__ void iface_flux(const double* c0, const double* c1, c
       pr[e] = pr[e] - 0.5 * ar;
     }
   }
-  if constexpr (!MHD) {
-    double cl, cr;
-    if constexpr (ORDER == 1) {  // cell values: sound speed from the ring
-      cl = c1[NEQ * Geo<ORDER>::PL];
-      cr = c2[NEQ * Geo<ORDER>::PL];
-    } else {
-      cl = sound_nr(ph.gamma * pl[4], pl[0]);
-      cr = sound_nr(ph.gamma * pr[4], pr[0]);
-    }
-    if constexpr (SOLVER == WX_SOLVER_HLLC) riemann_hllc_c<NEQ>(pl, pr, cl, cr, fx, ph.cv);
-    else riemann_hll_c<NEQ>(pl, pr, cl, cr, fx, ph.cv);
-  } else {
 #pragma unroll
-    for (int e = 0; e < NEQ; ++e) fx[e] = 0.0;
-    riemann_mhd<NEQ, SOLVER>(pl, pr, fx, ph.gamma, ph.cv);
-  }
+  for (int e = 0; e < NEQ; ++e) fx[e] = 0.0;
+  riemann_mhd<NEQ, SOLVER>(pl, pr, fx, ph.gamma, ph.cv);
 #pragma unroll
-  for (int e = 0; e < NEQ; ++e) f[perm<DIR, MHD>(e)] = fx[e];
+  for (int e = 0; e < NEQ; ++e) f[perm<DIR, true>(e)] = fx[e];
 }
 
 // Stores the result of the fused viscous step for one cell, counts
@@ -203,28 +186,24 @@ __device__ __forceinline__ void visc_store(const StageParams& P, const DevBlock&
 // Loads plane kk of the slab into its ring slot as primitives: the 16x16
 // physical cells, plus -- for the planes that get x/y fluxes -- the x/y ghost
 // frame (two deep for the second-order stage), gathered from the neighbours.
-// Converts one cell's conserved variables to primitives (plus, for the
-// first-order hydro stage, its sound speed) into ring plane pl,
+// Converts one cell's conserved variables to primitives into ring plane pl,
 // counting the flow2prim floors of physical cells when `count`.
-template <int NEQ, bool MHD, int ORDER, int CH>
+template <int NEQ, int ORDER>
 __device__ __forceinline__ void store_cell(const PhysParams& ph, double* pl, int i, int j, const double* u, bool count,
                                            unsigned* cnt) {
-  double p[NEQ], rinv;
-  const int st = flow2prim<NEQ, MHD>(u, p, ph.inv_cv, &rinv);
-  if constexpr (CH > NEQ) {
-    pl[NEQ * Geo<ORDER>::PL + hidx<ORDER>(i, j)] = sqrt_nr(ph.gamma * p[4] * rinv);
-  }
+  double p[NEQ];
+  const int st = flow2prim<NEQ, true>(u, p, ph.inv_cv);
   if (count && st != 0) atomicAdd(&cnt[st == 1 ? 0 : (st == 2 ? 1 : 2)], 1u);
 #pragma unroll
   for (int e = 0; e < NEQ; ++e) pl[e * Geo<ORDER>::PL + hidx<ORDER>(i, j)] = p[e];
 }
 
-template <int NEQ, bool MHD, int ORDER, int CH>
+template <int NEQ, int ORDER>
 __device__ __forceinline__ void load_plane(const StageParams& P, const DevBlock& B, int slot, int kk, int z0, int z1,
                                            double* ring, unsigned* cnt, bool skip_interior = false) {
   const int t = threadIdx.x;
   const PhysParams& ph = P.ph;
-  double* pl = ring + ring_slot(kk) * CH * Geo<ORDER>::PL;
+  double* pl = ring + ring_slot(kk) * NEQ * Geo<ORDER>::PL;
   const bool inner = (kk >= 1 && kk <= NC);
   const bool frame = (kk >= z0 && kk <= z1);  // plane gets x/y fluxes
   const int nframe = frame ? (ORDER == 2 ? 128 : 64) : 0;
@@ -244,7 +223,7 @@ __device__ __forceinline__ void load_plane(const StageParams& P, const DevBlock&
     double u[NEQ];
     if (inner && c < PLANE) load_cell<NEQ>(P.src, slot, i, j, kk, u);
     else gather_ghost<NEQ>(P.gsrc ? P.gsrc : P.src, B, slot, i, j, kk, u);
-    store_cell<NEQ, MHD, ORDER, CH>(ph, pl, i, j, u, c < PLANE && inner && frame, cnt);
+    store_cell<NEQ, ORDER>(ph, pl, i, j, u, c < PLANE && inner && frame, cnt);
     if (ORDER == 1 && P.gframe) {
       const int e = gframe_entry(kk, c);
       if (e >= 0) put_gframe<ORDER>(P.gframe, slot, e, pl, i, j);
@@ -266,12 +245,7 @@ __device__ __forceinline__ void load_plane(const StageParams& P, const DevBlock&
 // neighbours - 6 W) to plane m-1, whose z-neighbours are W(m-2) (still in
 // the buffer slot that W(m) replaces, read first by the same thread) and
 // W(m) (in registers).  The block-face z-neighbours are UP ghosts as well.
-// Two CTAs per SM where the shared memory allows it; registers are then
-// capped at 96 per thread (ten warps per CTA, five on each sub-partition).
-template <int NEQ, bool MHD, int ORDER, bool VISC>
-__host__ __device__ constexpr int stage_ctas_per_sm() {
-  return (!MHD && 2 * (stage_smem_bytes<NEQ, MHD, ORDER, VISC>() + 1024) <= 228 * 1024) ? 2 : 1;
-}
+// One CTA per SM (168 registers, 105-200 KB of shared memory).
 
 // Cell-centred electric field E = -v x B of the stage primitives at one ring
 // cell: the field-interpolated E of the field-CD scheme (Toth 2000, J. Comput.
@@ -286,18 +260,17 @@ __device__ __forceinline__ void efield(const double* c, double* E) {
   E[2] = v2 * b1 - v1 * b2;
 }
 
-template <int NEQ, bool MHD, int SOLVER, int ORDER, int LIM, bool VISC = false>
-__global__ void __launch_bounds__(STAGE_THREADS, (stage_ctas_per_sm<NEQ, MHD, ORDER, VISC>())) stage_kernel(StageParams P) {
-  constexpr int CH = ring_channels<NEQ, MHD, ORDER>();
+template <int NEQ, int SOLVER, int ORDER, int LIM, bool VISC = false>
+__global__ void __launch_bounds__(STAGE_THREADS, 1) stage_kernel(StageParams P) {
   extern __shared__ __align__(16) double smem[];
-  double* ring = smem;                                   // [RING][CH][Geo<ORDER>::PL]
-  double* fxs = ring + RING * CH * Geo<ORDER>::PL;               // [NEQ][16 rows][17]
+  double* ring = smem;                                   // [RING][NEQ][Geo<ORDER>::PL]
+  double* fxs = ring + RING * NEQ * Geo<ORDER>::PL;               // [NEQ][16 rows][17]
   double* fys = fxs + NEQ * 17 * NC;                     // [NEQ][17][16 cols]
   double* wpl = fys + NEQ * 17 * NC;                     // VISC: [2][NEQ][VPLANE]
   DevBlock& B = *reinterpret_cast<DevBlock*>(wpl + (VISC ? 2 * NEQ * VPLANE : 0));
   StageConsts& K = *reinterpret_cast<StageConsts*>(&B + 1);
   auto vq = [](int i, int j) { return i + (NC + 2) * j; };
-  Cfl<NEQ, MHD> cfl;
+  Cfl<NEQ, true> cfl;
   const int t = threadIdx.x;
   const int planes = NC / P.zsplit;
   const PhysParams& ph = P.ph;
@@ -328,17 +301,17 @@ __global__ void __launch_bounds__(STAGE_THREADS, (stage_ctas_per_sm<NEQ, MHD, OR
 
     // ---- prologue: planes z0-ORDER .. z0+ORDER-1, the z-interface z0-1/2,
     // then plane z0+ORDER into the slot of plane z0-ORDER ------------------
-    for (int kk = z0 - ORDER; kk <= z0 + ORDER - 1; ++kk) load_plane<NEQ, MHD, ORDER, CH>(P, B, slot, kk, z0, z1, ring, K.cnt);
+    for (int kk = z0 - ORDER; kk <= z0 + ORDER - 1; ++kk) load_plane<NEQ, ORDER>(P, B, slot, kk, z0, z1, ring, K.cnt);
     __syncthreads();
     if (t < PLANE) {
       const int m = z0 - 1;
-      const double* c0 = ring + ring_slot(m - 1) * CH * Geo<ORDER>::PL + hc;
-      const double* c1 = ring + ring_slot(m) * CH * Geo<ORDER>::PL + hc;
-      const double* c2 = ring + ring_slot(m + 1) * CH * Geo<ORDER>::PL + hc;
-      const double* c3 = ring + ring_slot(m + 2) * CH * Geo<ORDER>::PL + hc;
-      iface_flux<NEQ, MHD, SOLVER, ORDER, LIM, 2, true>(c0, c1, c2, c3, ph, znew, zslope, true);
-      if (MHD) bz_below = c1[7 * Geo<ORDER>::PL];
-      if (MHD && ph.flux_cd) efield<ORDER>(c1, e_below);
+      const double* c0 = ring + ring_slot(m - 1) * NEQ * Geo<ORDER>::PL + hc;
+      const double* c1 = ring + ring_slot(m) * NEQ * Geo<ORDER>::PL + hc;
+      const double* c2 = ring + ring_slot(m + 1) * NEQ * Geo<ORDER>::PL + hc;
+      const double* c3 = ring + ring_slot(m + 2) * NEQ * Geo<ORDER>::PL + hc;
+      iface_flux<NEQ, SOLVER, ORDER, LIM, 2, true>(c0, c1, c2, c3, ph, znew, zslope, true);
+      bz_below = c1[7 * Geo<ORDER>::PL];
+      if (ph.flux_cd) efield<ORDER>(c1, e_below);
     }
 #pragma unroll
     for (int e = 0; e < NEQ; ++e) zprev[e] = znew[e];
@@ -349,7 +322,7 @@ __global__ void __launch_bounds__(STAGE_THREADS, (stage_ctas_per_sm<NEQ, MHD, OR
       for (int e = 0; e < NEQ; ++e) wpl[((z0 - 1) & 1) * NEQ * VPLANE + e * VPLANE + vq(ci, cj)] = g[e];
     }
     __syncthreads();
-    load_plane<NEQ, MHD, ORDER, CH>(P, B, slot, z0 + ORDER, z0, z1, ring, K.cnt);
+    load_plane<NEQ, ORDER>(P, B, slot, z0 + ORDER, z0, z1, ring, K.cnt);
     __syncthreads();
 
     for (int m = z0; m <= z1; ++m) {
@@ -374,7 +347,7 @@ __global__ void __launch_bounds__(STAGE_THREADS, (stage_ctas_per_sm<NEQ, MHD, OR
         if (kl >= 1 && kl <= NC) load_cell<NEQ>(P.src, slot, ci, cj, kl, ul);
         else gather_ghost<NEQ>(P.gsrc ? P.gsrc : P.src, B, slot, ci, cj, kl, ul);
       }
-      if (kl <= z1 + ORDER) load_plane<NEQ, MHD, ORDER, CH>(P, B, slot, kl, z0, z1, ring, K.cnt, true);
+      if (kl <= z1 + ORDER) load_plane<NEQ, ORDER>(P, B, slot, kl, z0, z1, ring, K.cnt, true);
       // one-deep x/y frame of W(m): UP ghosts of plane m, on threads 256..319,
       // which compute no z-flux and at most one x/y interface pair
       if (VISC && t >= PLANE && t < PLANE + 4 * NC) {
@@ -390,7 +363,7 @@ __global__ void __launch_bounds__(STAGE_THREADS, (stage_ctas_per_sm<NEQ, MHD, OR
         }
       }
       if (t < 17 * NC) {
-        const double* pp = ring + ring_slot(m) * CH * Geo<ORDER>::PL;
+        const double* pp = ring + ring_slot(m) * NEQ * Geo<ORDER>::PL;
         // x-interface between ii and ii+1 in row jx: a half-warp takes 16
         // consecutive interfaces of one row (conflict-free shared loads),
         // threads 256..271 the last interface of each row; y-interface
@@ -399,28 +372,28 @@ __global__ void __launch_bounds__(STAGE_THREADS, (stage_ctas_per_sm<NEQ, MHD, OR
         const int iy = (t & 15) + 1, jj = t >> 4;
         {
           double f[NEQ];
-          iface_flux<NEQ, MHD, SOLVER, ORDER, LIM, 0>(pp + hidx<ORDER>(ii - 1, jx), pp + hidx<ORDER>(ii, jx), pp + hidx<ORDER>(ii + 1, jx),
+          iface_flux<NEQ, SOLVER, ORDER, LIM, 0>(pp + hidx<ORDER>(ii - 1, jx), pp + hidx<ORDER>(ii, jx), pp + hidx<ORDER>(ii + 1, jx),
                                                  pp + hidx<ORDER>(ii + 2, jx), ph, f);
 #pragma unroll
           for (int e = 0; e < NEQ; ++e) fxs[(e * NC + (jx - 1)) * 17 + ii] = f[e];
         }
         {
           double f[NEQ];
-          iface_flux<NEQ, MHD, SOLVER, ORDER, LIM, 1>(pp + hidx<ORDER>(iy, jj - 1), pp + hidx<ORDER>(iy, jj), pp + hidx<ORDER>(iy, jj + 1),
+          iface_flux<NEQ, SOLVER, ORDER, LIM, 1>(pp + hidx<ORDER>(iy, jj - 1), pp + hidx<ORDER>(iy, jj), pp + hidx<ORDER>(iy, jj + 1),
                                                  pp + hidx<ORDER>(iy, jj + 2), ph, f);
 #pragma unroll
           for (int e = 0; e < NEQ; ++e) fys[(e * 17 + jj) * NC + (iy - 1)] = f[e];
         }
       }
       if (t < PLANE) {  // z-flux m+1/2 last: znew is live only from here to phase B
-        const double* c1 = ring + ring_slot(m) * CH * Geo<ORDER>::PL + hc;
-        const double* c2 = ring + ring_slot(m + 1) * CH * Geo<ORDER>::PL + hc;
-        const double* c3 = ring + ring_slot(m + 2) * CH * Geo<ORDER>::PL + hc;
-        iface_flux<NEQ, MHD, SOLVER, ORDER, LIM, 2, true>(nullptr, c1, c2, c3, ph, znew, zslope, false);
+        const double* c1 = ring + ring_slot(m) * NEQ * Geo<ORDER>::PL + hc;
+        const double* c2 = ring + ring_slot(m + 1) * NEQ * Geo<ORDER>::PL + hc;
+        const double* c3 = ring + ring_slot(m + 2) * NEQ * Geo<ORDER>::PL + hc;
+        iface_flux<NEQ, SOLVER, ORDER, LIM, 2, true>(nullptr, c1, c2, c3, ph, znew, zslope, false);
       }
       if (late) {
-        double* pl = ring + ring_slot(kl) * CH * Geo<ORDER>::PL;
-        store_cell<NEQ, MHD, ORDER, CH>(ph, pl, ci, cj, ul, kl >= 1 && kl <= NC && kl >= z0 && kl <= z1, K.cnt);
+        double* pl = ring + ring_slot(kl) * NEQ * Geo<ORDER>::PL;
+        store_cell<NEQ, ORDER>(ph, pl, ci, cj, ul, kl >= 1 && kl <= NC && kl >= z0 && kl <= z1, K.cnt);
         if (ORDER == 1 && P.gframe && kl == NC + 1) put_gframe<ORDER>(P.gframe, slot, gframe_entry(kl, t), pl, ci, cj);
       }
       __syncthreads();
@@ -429,9 +402,9 @@ __global__ void __launch_bounds__(STAGE_THREADS, (stage_ctas_per_sm<NEQ, MHD, OR
         double s[NEQ];
 #pragma unroll
         for (int e = 0; e < NEQ; ++e) s[e] = 0.0;
-        if (MHD && ph.eight_wave) {  // Powell source (sources.f90:38-95) on the stage primitives
-          const double* pm = ring + ring_slot(m) * CH * Geo<ORDER>::PL;
-          const double* pu = ring + ring_slot(m + 1) * CH * Geo<ORDER>::PL;
+        if (ph.eight_wave) {  // Powell source (sources.f90:38-95) on the stage primitives
+          const double* pm = ring + ring_slot(m) * NEQ * Geo<ORDER>::PL;
+          const double* pu = ring + ring_slot(m + 1) * NEQ * Geo<ORDER>::PL;
           const int h = hc;
           const double divB = (pm[5 * Geo<ORDER>::PL + h + 1] - pm[5 * Geo<ORDER>::PL + h - 1]) / (2. * B.dx) +
                               (pm[6 * Geo<ORDER>::PL + h + Geo<ORDER>::W] - pm[6 * Geo<ORDER>::PL + h - Geo<ORDER>::W]) / (2. * B.dy) +
@@ -446,20 +419,20 @@ __global__ void __launch_bounds__(STAGE_THREADS, (stage_ctas_per_sm<NEQ, MHD, OR
           s[6] = -divB * v2;
           s[7] = -divB * v3;
         }
-        if (MHD) bz_below = ring[ring_slot(m) * CH * Geo<ORDER>::PL + 7 * Geo<ORDER>::PL + hc];
+        bz_below = ring[ring_slot(m) * NEQ * Geo<ORDER>::PL + 7 * Geo<ORDER>::PL + hc];
         const size_t o = cell_off(slot, NEQ, 0, ci, cj, m);
         // field-CD (brio-wu/flux_cd.f90:74-84): B from the central differences
         // of E over the six face neighbours; E of plane m-1 is carried
         double bcd[3] = {0.0, 0.0, 0.0};
-        if (MHD && ph.flux_cd) {
+        if (ph.flux_cd) {
           constexpr int PL = Geo<ORDER>::PL, W = Geo<ORDER>::W;
-          const double* pm = ring + ring_slot(m) * CH * PL + hc;
+          const double* pm = ring + ring_slot(m) * NEQ * PL + hc;
           double xl[3], xr[3], yl[3], yr[3], zu[3], ec[3];
           efield<ORDER>(pm - 1, xl);
           efield<ORDER>(pm + 1, xr);
           efield<ORDER>(pm - W, yl);
           efield<ORDER>(pm + W, yr);
-          efield<ORDER>(ring + ring_slot(m + 1) * CH * PL + hc, zu);
+          efield<ORDER>(ring + ring_slot(m + 1) * NEQ * PL + hc, zu);
           efield<ORDER>(pm, ec);
           const double hx = 0.5 * K.dtdx, hy = 0.5 * K.dtdy, hz = 0.5 * K.dtdz;
           bcd[0] = __ldg(P.base + o + 5 * (size_t)BCELLS) - hy * (yr[2] - yl[2]) - hz * (-zu[1] + e_below[1]);
@@ -476,8 +449,8 @@ __global__ void __launch_bounds__(STAGE_THREADS, (stage_ctas_per_sm<NEQ, MHD, OR
           const double fyl = fys[(e * 17 + cj - 1) * NC + ci - 1], fyr = fys[(e * 17 + cj) * NC + ci - 1];
           double v = __ldg(P.base + o + (size_t)e * BCELLS) + dtdx * (fxl - fxr) + dtdy * (fyl - fyr) +
                      dtdz * (zprev[e] - znew[e]);
-          if (MHD && ph.eight_wave) v = v + P.ctl->dt * P.dt_factor * s[e];
-          if (MHD && ph.flux_cd && e >= 5 && e <= 7) v = bcd[e - 5];
+          if (ph.eight_wave) v = v + P.ctl->dt * P.dt_factor * s[e];
+          if (ph.flux_cd && e >= 5 && e <= 7) v = bcd[e - 5];
           if (VISC) wv[e] = v;
           else P.out[o + (size_t)e * BCELLS] = v;
         }
@@ -493,7 +466,7 @@ __global__ void __launch_bounds__(STAGE_THREADS, (stage_ctas_per_sm<NEQ, MHD, OR
               un[e] = c + ph.eta * (+pe[vq(ci + 1, cj)] + pe[vq(ci - 1, cj)] + pe[vq(ci, cj + 1)] + pe[vq(ci, cj - 1)] +
                                     wv[e] + wb[e * VPLANE + vq(ci, cj)] - 6.0 * c);
             }
-            visc_store<NEQ, MHD>(P, B, un, o - NC * NC, cfl, K);
+            visc_store<NEQ, true>(P, B, un, o - NC * NC, cfl, K);
           }
 #pragma unroll
           for (int e = 0; e < NEQ; ++e) wb[e * VPLANE + vq(ci, cj)] = wv[e];
@@ -515,7 +488,7 @@ __global__ void __launch_bounds__(STAGE_THREADS, (stage_ctas_per_sm<NEQ, MHD, OR
         un[e] = c + ph.eta * (+pe[vq(ci + 1, cj)] + pe[vq(ci - 1, cj)] + pe[vq(ci, cj + 1)] + pe[vq(ci, cj - 1)] + g[e] +
                               wb[e * VPLANE + vq(ci, cj)] - 6.0 * c);
       }
-      visc_store<NEQ, MHD>(P, B, un, cell_off(slot, NEQ, 0, ci, cj, z1), cfl, K);
+      visc_store<NEQ, true>(P, B, un, cell_off(slot, NEQ, 0, ci, cj, z1), cfl, K);
     }
     // items past the first wave go, in list order, to whichever CTA
     // finishes first (the counter is zeroed before each launch): blocks at
@@ -789,6 +762,355 @@ __global__ void __launch_bounds__(STAGE_THREADS, 2) predictor_kernel(StageParams
     __syncthreads();
     w = K.next;
   }
+  __syncthreads();
+  if (t < 4 && K.cnt[t]) atomicAdd(&P.ctl->cnt[t], (unsigned long long)K.cnt[t]);
+}
+
+// ---------------------------------------------------------------------------
+// Second-order stage of the hydro equations (the corrector), laid out as the
+// predictor above: columns in registers, block-face interfaces on warps 8
+// and 9, one barrier per plane.  Shared memory holds two planes of
+// primitives with their one-deep x/y frame.  A column thread
+//  - limits its own x-slope and passes the state at its left face to the
+//    lane below by a shuffle, so every x-slope is computed once;
+//  - limits its own and the next row's y-slope;
+//  - limits the z-slope of the cell above, whose upper-face state it carries
+//    to the next plane's interface; the cell two planes up stays in
+//    registers until it is needed as a plane;
+//  - takes its next source and base cells by asynchronous copies.
+// A face thread keeps both ghost layers of its (side, row) in registers,
+// leaves the inner one in the frame for the slopes next to the face, and
+// solves the block-face interface.
+//
+// VISC (whole blocks) fuses doViscousStep (hydro_solver.f90:217-250): the
+// result W of plane m goes to one of two shared planes framed by the
+// half-step UP ghosts, and the update of plane m applies
+// U = W + eta (sum of the six neighbours - 6 W) to plane m-1, whose
+// z-neighbours are W(m-2) (in the place that W(m) takes, read first by the
+// same thread) and W(m).
+//
+// Bound, as the predictor, by the shared-memory data path (60 % busy) and
+// instruction issue (50 %) at ten warps per scheduler pair; two CTAs per SM
+// up to six equations need both 96 registers without spills (a plane is
+// converted in place at its z-interface instead of waiting in registers) and
+// at most 113 KB: at six equations the frame rows are unpadded for that.
+// 11,600-block AMR blast, five equations: fused 3.44 -> 2.87 ms, unfused
+// 2.72 -> 2.51 ms; 5,496-block winds mesh, six equations: fused (one CTA per
+// SM before) 2.37 -> 1.90 ms, unfused 1.55 -> 1.36 ms.  The prefetch of the
+// next base plane is 4 % of it; keeping the base in a shared plane instead
+// cost 15 % (less L1 for the ghost gathers).
+template <int NEQ, bool VISC>
+struct CorrSmem {
+  static constexpr int W = NC + 2;               // row of an 18-cell framed plane
+  static constexpr int PL = W * W;
+  double pl[3][NEQ][PL];                         // primitives of planes m, m+1; conserved, then
+                                                 // primitive variables of plane m+2
+  double fy[2][NEQ][(NC + 1) * NC];              // y-flux below row j (rows 0 and 16: block faces)
+  double ex[2][2][NEQ][NC];                      // x-flux of the low and the high block face
+  double w[VISC ? 2 : 1][VISC ? NEQ : 1][VISC ? PL : 1];  // W of planes m, m-1, framed by UP ghosts
+  double wg[VISC ? 2 : 1][NEQ][VISC ? 4 * NC : 1];  // the frame's UP ghosts, a plane ahead
+  DevBlock B;
+  StageConsts K;
+};
+
+template <int D>
+struct Dir { static constexpr int value = D; };
+template <int NEQ>
+struct Flux {
+  double v[NEQ];
+  __device__ __forceinline__ explicit Flux(const double* f) {
+#pragma unroll
+    for (int e = 0; e < NEQ; ++e) v[e] = f[e];
+  }
+};
+
+// Flux between two face states already permuted to direction DIR.
+template <int NEQ, int SOLVER, int DIR>
+__device__ __forceinline__ void state_flux(const double* l, const double* r, const PhysParams& ph, double* f) {
+  const double cl = sound_nr(ph.gamma * l[4], l[0]);
+  const double cr = sound_nr(ph.gamma * r[4], r[0]);
+  double fx[NEQ];
+  if constexpr (SOLVER == WX_SOLVER_HLLC) riemann_hllc_c<NEQ>(l, r, cl, cr, fx, ph.cv);
+  else riemann_hll_c<NEQ>(l, r, cl, cr, fx, ph.cv);
+#pragma unroll
+  for (int e = 0; e < NEQ; ++e) f[perm<DIR, false>(e)] = fx[e];
+}
+
+template <int NEQ, bool VISC>
+__host__ __device__ constexpr int corr_ctas_per_sm() {
+  return 2 * (sizeof(CorrSmem<NEQ, VISC>) + 1024) <= 228 * 1024 ? 2 : 1;
+}
+
+template <int NEQ, int SOLVER, int LIM, bool VISC>
+__global__ void __launch_bounds__(STAGE_THREADS, (corr_ctas_per_sm<NEQ, VISC>())) corrector_kernel(StageParams P) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  CorrSmem<NEQ, VISC>& S = *reinterpret_cast<CorrSmem<NEQ, VISC>*>(smraw);
+  constexpr int W = CorrSmem<NEQ, VISC>::W, PL = CorrSmem<NEQ, VISC>::PL;
+  DevBlock& B = S.B;
+  StageConsts& K = S.K;
+  const int t = threadIdx.x, lane = t & (NC - 1);
+  const PhysParams& ph = P.ph;
+  const int planes = NC / P.zsplit;
+  const bool column = t < PLANE;
+  const int ci = lane + 1, cj = (t >> 4) + 1;                  // column threads
+  const int q = t - PLANE, side = q >> 4;                      // face threads: 0, 1 x; 2, 3 y
+  const bool high = side & 1;
+  const int gi = side == 0 ? 0 : (side == 1 ? NC + 1 : lane + 1);   // inner ghost
+  const int gj = side == 2 ? 0 : (side == 3 ? NC + 1 : lane + 1);
+  const int oi = side == 0 ? -1 : (side == 1 ? NC + 2 : lane + 1);  // outer ghost
+  const int oj = side == 2 ? -1 : (side == 3 ? NC + 2 : lane + 1);
+  const int h = column ? ci + W * cj : gi + W * gj;            // place in a framed plane
+  const double* gsrc = P.gsrc ? P.gsrc : P.src;
+  Cfl<NEQ, false> cfl;
+  if (t < 4) K.cnt[t] = 0;
+
+  for (int w = blockIdx.x; w < P.nwork;) {
+    const int slot = P.work[w / P.zsplit];
+    const int z0 = 1 + (w % P.zsplit) * planes, z1 = z0 + planes - 1;
+    __syncthreads();
+    if (t < (int)(sizeof(DevBlock) / 4)) reinterpret_cast<int*>(&B)[t] = reinterpret_cast<const int*>(P.blocks + slot)[t];
+    __syncthreads();
+    if (t == 0) {  // read after the prologue's barrier
+      const double dtp = P.ctl->dt * P.dt_factor;
+      K.dtdx = dtp / B.dx;
+      K.dtdy = dtp / B.dy;
+      K.dtdz = dtp / B.dz;
+      K.idx = 1.0 / B.dx;
+      K.idy = 1.0 / B.dy;
+      K.idz = 1.0 / B.dz;
+    }
+    if (column) {
+      // conserved variables of the column's cell in plane kk
+      auto load = [&](int kk, double* u) {
+        if (kk >= 1 && kk <= NC) load_cell<NEQ>(P.src, slot, ci, cj, kk, u);
+        else gather_ghost<NEQ>(gsrc, B, slot, ci, cj, kk, u);
+      };
+      // the same into the plane's place in shared memory, asynchronously where
+      // it is a plain copy; the thread itself converts it (to_plane)
+      auto fetch = [&](int kk) {
+        double* d = &S.pl[(unsigned)(kk + 3) % 3u][0][h];
+        if (kk >= 1 && kk <= NC) {
+          const double* g = P.src + cell_off(slot, NEQ, 0, ci, cj, kk);
+#pragma unroll
+          for (int e = 0; e < NEQ; ++e) copy_async8(d + e * PL, g + (size_t)e * BCELLS);
+        } else {
+          double u[NEQ];
+          gather_ghost<NEQ>(gsrc, B, slot, ci, cj, kk, u);
+#pragma unroll
+          for (int e = 0; e < NEQ; ++e) d[e * PL] = u[e];
+        }
+      };
+      auto to_prim = [&](int kk, const double* u, double* p) {
+        const int st = flow2prim<NEQ, false>(u, p, ph.inv_cv);
+        if (st != 0 && kk >= z0 && kk <= z1) atomicAdd(&K.cnt[st == 1 ? 0 : (st == 2 ? 1 : 2)], 1u);
+      };
+      auto to_plane = [&](int kk, double* p) {
+        double* d = &S.pl[(unsigned)(kk + 3) % 3u][0][h];
+        double u[NEQ];
+#pragma unroll
+        for (int e = 0; e < NEQ; ++e) u[e] = d[e * PL];
+        to_prim(kk, u, p);
+#pragma unroll
+        for (int e = 0; e < NEQ; ++e) d[e * PL] = p[e];
+      };
+      double lz[NEQ], zf[NEQ];
+      {  // planes z0-2 .. z0+1 and the z-interface z0-1/2; plane z0+2 on its way
+        double u[NEQ], p0[NEQ], p1[NEQ], pc[NEQ], pu[NEQ], l[NEQ], r[NEQ];
+        fetch(z0);
+        fetch(z0 + 1);
+        fetch(z0 + 2);
+        load(z0 - 2, u);
+        to_prim(z0 - 2, u, p0);
+        load(z0 - 1, u);
+        if (VISC) {  // W(z0-1) of the column: the bottom UP ghost
+#pragma unroll
+          for (int e = 0; e < NEQ; ++e) S.w[(z0 - 1) & 1][e][h] = u[e];
+        }
+        to_prim(z0 - 1, u, p1);
+        copy_async_wait();
+        to_plane(z0, pc);
+        to_plane(z0 + 1, pu);
+#pragma unroll
+        for (int e = 0; e < NEQ; ++e) {
+          const int k = perm<2, false>(e);
+          const double dm = pc[k] - p1[k];
+          l[e] = p1[k] + 0.5 * average_t<LIM>(p1[k] - p0[k], dm, ph.limiter);
+          const double s = average_t<LIM>(dm, pu[k] - pc[k], ph.limiter);
+          r[e] = pc[k] - 0.5 * s;
+          lz[e] = pc[k] + 0.5 * s;
+        }
+        state_flux<NEQ, SOLVER, 2>(l, r, ph, zf);
+      }
+      plane_barrier();
+
+      for (int m = z0; m <= z1; ++m) {
+        const int b = m & 1;
+        double dx[NEQ], dz[NEQ], f[NEQ], v[NEQ], pc[NEQ];
+        // the base plane after this one into L2 (16 lines per equation)
+        if (t < 16 * NEQ && m < z1) prefetch_l2(P.base + cell_off(slot, NEQ, t >> 4, 1, 1, m + 1) + (size_t)(t & 15) * 16);
+        const double* pp = &S.pl[(unsigned)m % 3u][0][h];
+#pragma unroll
+        for (int e = 0; e < NEQ; ++e) pc[e] = pp[e * PL];
+        {  // y-interface to row cj+1 (the last row's flux is a face thread's)
+          double l[NEQ], r[NEQ];
+          const int o2 = cj < NC ? 2 * W : W;
+#pragma unroll
+          for (int e = 0; e < NEQ; ++e) {
+            const int k = perm<1, false>(e);
+            const double a = pp[k * PL + W], dm = a - pc[k];
+            l[e] = pc[k] + 0.5 * average_t<LIM>(pc[k] - pp[k * PL - W], dm, ph.limiter);
+            r[e] = a - 0.5 * average_t<LIM>(dm, pp[k * PL + o2] - a, ph.limiter);
+          }
+          state_flux<NEQ, SOLVER, 1>(l, r, ph, f);
+          if (cj < NC) {
+#pragma unroll
+            for (int e = 0; e < NEQ; ++e) S.fy[b][e][cj * NC + lane] = f[e];
+          }
+        }
+        {  // x-interface to cell ci+1 (the last lane's flux is a face thread's)
+          double l[NEQ], r[NEQ];
+#pragma unroll
+          for (int e = 0; e < NEQ; ++e) {
+            const double s = average_t<LIM>(pc[e] - pp[e * PL - 1], pp[e * PL + 1] - pc[e], ph.limiter);
+            l[e] = pc[e] + 0.5 * s;
+            r[e] = __shfl_down_sync(0xffffffffu, pc[e] - 0.5 * s, 1, NC);
+          }
+          state_flux<NEQ, SOLVER, 0>(l, r, ph, f);
+#pragma unroll
+          for (int e = 0; e < NEQ; ++e) {
+            const double xl = __shfl_up_sync(0xffffffffu, f[e], 1, NC);
+            dx[e] = lane == 0 ? -f[e] : (lane == NC - 1 ? xl : xl - f[e]);
+          }
+        }
+        {  // z-interface m+1/2: the column's own cells
+          const double* pa = &S.pl[(unsigned)(m + 1) % 3u][0][h];
+          double l[NEQ], r[NEQ], pu[NEQ];
+          if (m > z0) copy_async_wait();
+          to_plane(m + 2, pu);
+#pragma unroll
+          for (int e = 0; e < NEQ; ++e) {
+            const int k = perm<2, false>(e);
+            const double a = pa[k * PL];
+            const double s = average_t<LIM>(a - pc[k], pu[k] - a, ph.limiter);
+            r[e] = a - 0.5 * s;
+            l[e] = lz[e];
+            lz[e] = a + 0.5 * s;
+          }
+          state_flux<NEQ, SOLVER, 2>(l, r, ph, f);
+#pragma unroll
+          for (int e = 0; e < NEQ; ++e) {
+            dz[e] = zf[e] - f[e];
+            zf[e] = f[e];
+          }
+        }
+        const size_t o = cell_off(slot, NEQ, 0, ci, cj, m);
+#pragma unroll
+        for (int e = 0; e < NEQ; ++e) v[e] = __ldg(P.base + o + (size_t)e * BCELLS);
+        plane_barrier();
+        // conservative update of plane m (godunov.f90:259-271); each
+        // direction's two fluxes are subtracted before they are scaled, so
+        // equal fluxes cancel exactly
+        const double dtdx = K.dtdx, dtdy = K.dtdy, dtdz = K.dtdz;
+        const bool xedge = lane == 0 || lane == NC - 1;
+        const double* ex = &S.ex[b][lane >> 3][0][cj - 1];
+#pragma unroll
+        for (int e = 0; e < NEQ; ++e) {
+          const double xe = xedge ? ex[e * NC] : 0.0;
+          const double ddx = dx[e] + (lane == 0 ? xe : -xe);
+          const double dy = S.fy[b][e][(cj - 1) * NC + lane] - S.fy[b][e][cj * NC + lane];
+          v[e] = v[e] + dtdx * ddx + dtdy * dy + dtdz * dz[e];
+          if (!VISC) P.out[o + (size_t)e * BCELLS] = v[e];
+        }
+        if (VISC) {  // W(m) over W(m-2) of the column, and the viscous step of plane m-1
+#pragma unroll
+          for (int e = 0; e < NEQ; ++e) {
+            const double* pw = &S.w[b ^ 1][e][h];
+            const double below = S.w[b][e][h];
+            S.w[b][e][h] = v[e];
+            v[e] = pw[0] + ph.eta * ((pw[1] + pw[-1]) + (pw[W] + pw[-W]) + (v[e] + below) - 6.0 * pw[0]);
+          }
+          if (m > z0) visc_store<NEQ, false>(P, B, v, o - NC * NC, cfl, K);
+        }
+        if (m < z1) fetch(m + 3);  // over plane m, which no one reads any more
+      }
+      if (VISC) {  // plane z1: above it, the top UP ghost
+        double g[NEQ], un[NEQ];
+        gather_ghost<NEQ>(gsrc, B, slot, ci, cj, z1 + 1, g);
+        plane_barrier();
+#pragma unroll
+        for (int e = 0; e < NEQ; ++e) {
+          const double* pw = &S.w[z1 & 1][e][h];
+          un[e] = pw[0] + ph.eta * ((pw[1] + pw[-1]) + (pw[W] + pw[-W]) + (g[e] + S.w[(z1 - 1) & 1][e][h]) - 6.0 * pw[0]);
+        }
+        visc_store<NEQ, false>(P, B, un, cell_off(slot, NEQ, 0, ci, cj, z1), cfl, K);
+      }
+    } else {
+      double g2[NEQ];  // primitives of the outer ghost; the inner one's are in the frame
+      auto take = [&](int kk, const double* u1, const double* u2) {
+        double g1[NEQ];
+        flow2prim<NEQ, false>(u1, g1, ph.inv_cv);
+        flow2prim<NEQ, false>(u2, g2, ph.inv_cv);
+#pragma unroll
+        for (int e = 0; e < NEQ; ++e) {
+          S.pl[(unsigned)kk % 3u][e][h] = g1[e];
+          if (VISC) S.wg[kk & 1][e][q] = u1[e];
+        }
+      };
+      // face state of the block-face interface from its four cells in order
+      auto faces = [&](const double* pg, int step, auto dir) {
+        constexpr int DIR = decltype(dir)::value;
+        double l[NEQ], r[NEQ], f[NEQ];
+#pragma unroll
+        for (int e = 0; e < NEQ; ++e) {
+          const int k = perm<DIR, false>(e);
+          const double g = pg[k * PL], a = pg[k * PL + step], a2 = pg[k * PL + 2 * step];
+          const double c0 = high ? a2 : g2[k], c1 = high ? a : g, c2 = high ? g : a, c3 = high ? g2[k] : a2;
+          const double dm = c2 - c1;
+          l[e] = c1 + 0.5 * average_t<LIM>(c1 - c0, dm, ph.limiter);
+          r[e] = c2 - 0.5 * average_t<LIM>(dm, c3 - c2, ph.limiter);
+        }
+        state_flux<NEQ, SOLVER, DIR>(l, r, ph, f);
+        return Flux<NEQ>(f);
+      };
+      {
+        double u1[NEQ], u2[NEQ];
+        gather_ghost<NEQ>(gsrc, B, slot, gi, gj, z0, u1);
+        gather_ghost<NEQ>(gsrc, B, slot, oi, oj, z0, u2);
+        take(z0, u1, u2);
+      }
+      plane_barrier();
+      for (int m = z0; m <= z1; ++m) {
+        const int b = m & 1;
+        if (side < 2) {
+          const Flux<NEQ> f = faces(&S.pl[(unsigned)m % 3u][0][h], high ? -1 : 1, Dir<0>());
+#pragma unroll
+          for (int e = 0; e < NEQ; ++e) S.ex[b][side][e][lane] = f.v[e];
+        } else {
+          const Flux<NEQ> f = faces(&S.pl[(unsigned)m % 3u][0][h], high ? -W : W, Dir<1>());
+#pragma unroll
+          for (int e = 0; e < NEQ; ++e) S.fy[b][e][(high ? NC * NC : 0) + lane] = f.v[e];
+        }
+        if (m < z1) {
+          double u1[NEQ], u2[NEQ];
+          gather_ghost<NEQ>(gsrc, B, slot, gi, gj, m + 1, u1);
+          gather_ghost<NEQ>(gsrc, B, slot, oi, oj, m + 1, u2);
+          take(m + 1, u1, u2);
+        }
+        plane_barrier();
+        if (VISC) {
+#pragma unroll
+          for (int e = 0; e < NEQ; ++e) S.w[b][e][h] = S.wg[b][e][q];
+        }
+      }
+      if (VISC) plane_barrier();
+    }
+    // items past the first wave go, in list order, to whichever CTA
+    // finishes first (the counter is zeroed before each launch)
+    if (t == 0) K.next = (int)gridDim.x + (int)atomicAdd(&P.ctl->work_next[1], 1u);
+    __syncthreads();
+    w = K.next;
+  }
+  if (VISC && P.do_dt) block_min_dt(cfl.dt(), P.ctl);
   __syncthreads();
   if (t < 4 && K.cnt[t]) atomicAdd(&P.ctl->cnt[t], (unsigned long long)K.cnt[t]);
 }
