@@ -1377,15 +1377,62 @@ int wx3d_set_dtmin(wx_ctx* c, double v) {
   return WX_OK;
 }
 
+// Whether [p, p + bytes) lies inside one allocation on the device (false
+// where that cannot be told).
+static bool device_range(int dev, const void* p, size_t bytes) {
+  using AddressRange = int (*)(unsigned long long*, size_t*, unsigned long long);
+  static const AddressRange range = [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      f = nullptr;
+    return reinterpret_cast<AddressRange>(f);
+  }();
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  if (at.type != cudaMemoryTypeDevice || at.device != dev || !range) return false;
+  unsigned long long base = 0;
+  size_t size = 0;
+  const unsigned long long a = reinterpret_cast<unsigned long long>(p);
+  return range(&base, &size, a) == 0 && a >= base && a + bytes <= base + size;
+}
+
 static int copy_blocks(wx_ctx* c, int32_t array, int32_t n, const int32_t* slots, double* buf, bool pack) {
   if (!c || n < 0 || (n > 0 && (!slots || !buf)) || (array != 0 && array != 1)) return WX_ERR_INVALID_ARG;
-  double* a = array == 0 ? c->dU : c->dUP;
-  const size_t per = (size_t)c->neq * BCELLS * 8;
-  for (int b = 0; b < n; ++b) {
+  for (int b = 0; b < n; ++b)
     if (slots[b] < 0 || slots[b] >= c->max_blocks) return fail(c, WX_ERR_INVALID_ARG, "slot %d out of range", slots[b]);
-    double* s = a + (size_t)slots[b] * c->neq * BCELLS;
-    double* d = buf + (size_t)b * c->neq * BCELLS;
-    WX_CUDA(cudaMemcpyAsync(pack ? d : s, pack ? s : d, per, cudaMemcpyDeviceToDevice, c->stream));
+  double* a = array == 0 ? c->dU : c->dUP;
+  const size_t block = (size_t)c->neq * BCELLS;
+  // the kernel takes 16-byte aligned buffers that lie in one allocation of
+  // this context's device, and each slot once when it writes them; other
+  // calls copy block by block, in order, with the copies' own checks
+  bool one_launch = n > 0 && reinterpret_cast<uintptr_t>(buf) % 16 == 0 && device_range(c->dev, buf, block * 8 * (size_t)n);
+  if (one_launch && !pack) {
+    std::vector<char> seen(c->max_blocks, 0);
+    for (int b = 0; b < n; ++b) {
+      if (seen[slots[b]]) one_launch = false;
+      seen[slots[b]] = 1;
+    }
+  }
+  if (one_launch) {
+    for (int o = 0; o < n; o += COPY_SLOTS) {
+      CopySlots cs;
+      const int m = std::min(COPY_SLOTS, n - o);
+      std::copy(slots + o, slots + o + m, cs.s);
+      copy_blocks_kernel<<<dim3((unsigned)(block / 2 / COPY_PIECE), m), 256, 0, c->stream>>>(a, cs, c->neq, buf + (size_t)o * block,
+                                                                                            pack ? 1 : 0);
+      WX_LAUNCHED();
+    }
+  } else {
+    for (int b = 0; b < n; ++b) {
+      double* s = a + (size_t)slots[b] * block;
+      double* d = buf + (size_t)b * block;
+      WX_CUDA(cudaMemcpyAsync(pack ? d : s, pack ? s : d, block * 8, cudaMemcpyDeviceToDevice, c->stream));
+    }
   }
   WX_CUDA(cudaStreamSynchronize(c->stream));
   return WX_OK;
