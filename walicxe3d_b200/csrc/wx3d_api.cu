@@ -45,6 +45,7 @@ struct Kern {
   size_t smem1 = 0;  // dynamic shared memory of the predictor and the corrector
   size_t smem2 = 0;
   size_t smem2v = 0;
+  size_t smemv = 0;  // of the viscous kernel
 };
 
 template <int NEQ, bool MHD, int SOLVER, int LIM>
@@ -67,6 +68,7 @@ Kern make_kern() {
   }
   k.lax = lax_kernel<NEQ, MHD>;
   k.visc = viscous_kernel<NEQ, MHD>;
+  k.smemv = sizeof(ViscSmem<NEQ>);
   k.dt = dt_kernel<NEQ, MHD>;
   k.wind = wind_kernel<NEQ, MHD>;
   k.src = source_kernel<NEQ, MHD>;
@@ -293,6 +295,7 @@ struct wx_ctx {
   double* dG = nullptr;
   bool mark_ghosts = false;       // the first-order stage writes dG
   bool g_step = false;            // the step being enqueued writes dG
+  int counters_zeroed = 0;        // stages (bits 1, 2) whose item counter the enqueued work leaves at zero
   bool g_valid = false;           // dG holds the ghosts of the state in dW (with prestep)
   cudaGraphExec_t graph = nullptr;
   bool graph_valid = false;
@@ -473,6 +476,7 @@ int set_stage_attrs(wx_ctx* c) {
   WX_CUDA(cudaFuncSetAttribute(c->k.stage1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->k.smem1));
   WX_CUDA(cudaFuncSetAttribute(c->k.stage2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->k.smem2));
   WX_CUDA(cudaFuncSetAttribute(c->k.stage2v, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->k.smem2v));
+  WX_CUDA(cudaFuncSetAttribute(c->k.visc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)c->k.smemv));
   return WX_OK;
 }
 
@@ -482,7 +486,7 @@ int launch_dt(wx_ctx* c, const double* u) {
   ctl_reset_dtmin_kernel<<<1, 1, 0, c->stream>>>(c->dCtl);
   WX_LAUNCHED();
   DtParams P{u, c->dBlocks, c->dWork, c->nwork, c->dCtl, c->ph};
-  c->k.dt<<<grid_for(c, (const void*)c->k.dt, 256, 0, c->nwork), 256, 0, c->stream>>>(P);
+  c->k.dt<<<grid_for(c, (const void*)c->k.dt, 256, 0, c->nwork * (NC / DT_PLANES)), 256, 0, c->stream>>>(P);
   WX_LAUNCHED();
   return WX_OK;
 }
@@ -505,7 +509,11 @@ int launch_stage(wx_ctx* c, int order, const double* src, const double* base, do
   const size_t smem = order == 1 ? c->k.smem1 : (fused ? c->k.smem2v : c->k.smem2);
   const int grid = grid_for(c, (const void*)fn, STAGE_THREADS, smem, c->nwork * c->zsplit);
   const int kind = (order == 2 || factor == 1.0) ? 1 : 0;
-  WX_CUDA(cudaMemsetAsync(&c->dCtl->work_next[order - 1], 0, sizeof(unsigned), c->stream));
+  // the step's first kernel zeroes both stages' item counters; launches
+  // outside that sequence (the autotuner's, repeated parts) do it themselves
+  if (!(c->counters_zeroed & order))
+    WX_CUDA(cudaMemsetAsync(&c->dCtl->work_next[order - 1], 0, sizeof(unsigned), c->stream));
+  c->counters_zeroed &= ~order;
   tick(c, kind, true);
   fn<<<grid, STAGE_THREADS, smem, c->stream>>>(P);
   WX_LAUNCHED();
@@ -513,13 +521,33 @@ int launch_stage(wx_ctx* c, int order, const double* src, const double* base, do
   return WX_OK;
 }
 
+// One CTA per block; where that leaves SMs without their three CTAs, a
+// cluster of up to eight CTAs splits each block's planes.
+cudaError_t launch_viscous(const Kern& k, ViscParams V, int nwork, int nsm, cudaStream_t s) {
+  V.zsplit = 1;
+  while (V.zsplit < 8 && nwork * V.zsplit < 3 * nsm) V.zsplit *= 2;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(nwork * V.zsplit));
+  cfg.blockDim = dim3(STAGE_THREADS);
+  cfg.dynamicSmemBytes = k.smemv;
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = V.zsplit;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = V.zsplit > 1 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, k.visc, V);
+}
+
 // doViscousStep in place on w (the stage result), UP ghosts (zero for
 // single-stage solvers)
 int launch_visc(wx_ctx* c, int zero_ghost, double* w = nullptr) {
-  ViscParams V{w ? w : c->dW, c->dUP, c->dBlocks, c->dWork, c->nwork, zero_ghost, sources_on(c) ? 0 : 1, c->dCtl, c->ph};
+  ViscParams V{w ? w : c->dW, c->dUP, c->dBlocks, c->dWork, 0, zero_ghost, sources_on(c) ? 0 : 1, c->dCtl, c->ph};
+  if (c->nwork == 0) return WX_OK;
   tick(c, 2, true);
-  c->k.visc<<<grid_for(c, (const void*)c->k.visc, 256, 0, c->nwork), 256, 0, c->stream>>>(V);
-  WX_LAUNCHED();
+  WX_CUDA(launch_viscous(c->k, V, c->nwork, c->nsm, c->stream));
+  ++c->launches;
   tick(c, 2, false);
   return WX_OK;
 }
@@ -578,6 +606,7 @@ int enqueue_solver(wx_ctx* c, bool bump_it, bool finish_output) {
   step_begin_kernel<<<1, 1, 0, c->stream>>>(c->dCtl, c->ph.cfl, c->cfg.cooling_type != WX_COOL_NONE, c->ph.dtout,
                                             c->ph.t_sc, bump_it ? 1 : 0);
   WX_LAUNCHED();
+  c->counters_zeroed = 3;
   int rc;
   if (!c->hwind.empty()) {
     if (!c->wind_ready) return fail(c, WX_ERR_GENERIC, "wind sources without their redirected neighbour table");
@@ -1340,6 +1369,7 @@ int wx3d_step_part(wx_ctx* c, int32_t part) {
       step_begin_kernel<<<1, 1, 0, c->stream>>>(c->dCtl, c->ph.cfl, c->cfg.cooling_type != WX_COOL_NONE, c->ph.dtout,
                                                 c->ph.t_sc, 1);
       WX_LAUNCHED();
+      c->counters_zeroed = 3;
       return WX_OK;
     case 1: return solver_first(c);
     case 2: return solver_second(c, true);
@@ -2665,8 +2695,9 @@ extern "C" int wx3d_hydro_step_noalloc(const wx_config* cfg, int32_t nslots, con
   int32_t* dWork = reinterpret_cast<int32_t*>(base + NOALLOC_WORK_OFF);
   DevCtl* dCtl = reinterpret_cast<DevCtl*>(base + NOALLOC_CTL_OFF);
 
-  DevBlock hb[NOALLOC_MAX_BLOCKS];
-  int32_t work[NOALLOC_MAX_BLOCKS];
+  alignas(DevBlock) unsigned char host[NOALLOC_BYTES - NOALLOC_TABLE_OFF] = {};
+  DevBlock* hb = reinterpret_cast<DevBlock*>(host);
+  int32_t* work = reinterpret_cast<int32_t*>(host + (NOALLOC_WORK_OFF - NOALLOC_TABLE_OFF));
   int nwork = 0;
   if ((rc = noalloc_table(*cfg, nslots, local_blocks, hb, work, &nwork))) {
     std::fprintf(stderr, "wx3d_hydro_step_noalloc: invalid mesh\n");
@@ -2696,13 +2727,15 @@ extern "C" int wx3d_hydro_step_noalloc(const wx_config* cfg, int32_t nslots, con
   auto ck = [](cudaError_t e) { return e == cudaSuccess ? WX_OK : WX_ERR_CUDA; };
   if ((rc = ck(cudaFuncSetAttribute(k.stage1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem1)))) return rc;
   if ((rc = ck(cudaFuncSetAttribute(k.stage2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem2)))) return rc;
-  if ((rc = ck(cudaMemcpyAsync(dBlocks, hb, sizeof(DevBlock) * nslots, cudaMemcpyHostToDevice, s)))) return rc;
-  if ((rc = ck(cudaMemcpyAsync(dWork, work, 4 * (size_t)nwork, cudaMemcpyHostToDevice, s)))) return rc;
-  if ((rc = ck(cudaMemcpyAsync(dCtl, &h, sizeof(DevCtl), cudaMemcpyHostToDevice, s)))) return rc;
+  if ((rc = ck(cudaFuncSetAttribute(k.visc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smemv)))) return rc;
+  // the table, the work list and the control block lie one after the other
+  // in the scratch: one copy
+  std::memcpy(host + (NOALLOC_CTL_OFF - NOALLOC_TABLE_OFF), &h, sizeof(DevCtl));
+  if ((rc = ck(cudaMemcpyAsync(dBlocks, host, sizeof host, cudaMemcpyHostToDevice, s)))) return rc;
 
   // getTimestep on u_in, then the step sequence of enqueue_solver
   DtParams D{u_in, dBlocks, dWork, nwork, dCtl, ph};
-  k.dt<<<noalloc_grid((const void*)k.dt, 256, 0, nwork, nsm), 256, 0, s>>>(D);
+  k.dt<<<noalloc_grid((const void*)k.dt, 256, 0, nwork * (NC / DT_PLANES), nsm), 256, 0, s>>>(D);
   step_begin_kernel<<<1, 1, 0, s>>>(dCtl, ph.cfl, 0, ph.dtout, ph.t_sc, 1);
   const int solver = cfg->solver_type;
   int zero_ghost = 0;
@@ -2721,8 +2754,8 @@ extern "C" int wx3d_hydro_step_noalloc(const wx_config* cfg, int32_t nslots, con
     stage(k.stage1, k.smem1, u_in, dUP, 0.5);
     stage(k.stage2, k.smem2, dUP, u_out, 1.0);
   }
-  ViscParams V{u_out, dUP, dBlocks, dWork, nwork, zero_ghost, 1, dCtl, ph};
-  k.visc<<<noalloc_grid((const void*)k.visc, 256, 0, nwork, nsm), 256, 0, s>>>(V);
+  ViscParams V{u_out, dUP, dBlocks, dWork, 0, zero_ghost, 1, dCtl, ph};
+  if (nwork > 0 && (rc = ck(launch_viscous(k, V, nwork, nsm, s)))) return rc;
   step_end_kernel<<<1, 1, 0, s>>>(dCtl, 1);
   if ((rc = ck(cudaGetLastError()))) return rc;
   if ((rc = ck(cudaMemcpyAsync(&h, dCtl, sizeof(DevCtl), cudaMemcpyDeviceToHost, s)))) return rc;

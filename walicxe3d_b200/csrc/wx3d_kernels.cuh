@@ -542,6 +542,10 @@ struct PredSmem {
 
 // Barrier of all threads of a stage CTA, met by the roles at different places.
 __device__ __forceinline__ void plane_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(STAGE_THREADS) : "memory"); }
+// Barrier of all threads of the CTA's cluster.
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
 __device__ __forceinline__ void copy_async8(double* smem, const double* g) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(g) : "memory");
 }
@@ -1181,94 +1185,140 @@ struct ViscParams {
   const double* __restrict__ up;       // predictor state: source of the face ghosts
   const DevBlock* __restrict__ blocks;
   const int32_t* __restrict__ work;
-  int32_t nwork;
+  int32_t zsplit;                      // CTAs per block, one cluster (1, 2, 4 or 8)
   int32_t zero_ghost;                  // single-stage solvers: UP ghosts are never filled (0)
   int32_t do_dt;                       // fold the CFL minimum of the new state
   DevCtl* ctl;
   PhysParams ph;
 };
 
-// Four CTAs per SM (at most 64 registers): 2.87 instead of 3.05 ms per
-// step on the 20,896-block winds mesh with three.
+// One CTA per block, or a cluster of S CTAs that split its planes where the
+// mesh has too few blocks (launch_viscous).  HBM-bound: W is read and written
+// once, the ghosts of UP once.  Columns copy their cells a few planes ahead
+// into a ring of shared planes (no registers held while a load is in flight)
+// and warps 8 and 9 gather the frame from UP a plane ahead, so three CTAs per
+// SM keep about 60 KB of loads in flight; one barrier per plane.  The update
+// is in place: the planes just outside a slab are read before the cluster's
+// barrier, and the first write follows it.  11,600 blocks of five equations:
+// 1.57 -> 1.02 ms (the x-face ghosts cost a 32-byte sector per cell: with
+// them 5.1 GB, 0.79 ms at the copy rate); 20,896 blocks of six: 2.87 -> 2.32
+// ms.  64 blocks in clusters of eight: 26 -> 16 us; 16 MHD blocks: 54 -> 14.
+constexpr int VRING = 4;
+template <int NEQ>
+struct ViscSmem {
+  double pl[VRING][NEQ][VPLANE];   // planes of W with the one-deep ghost frame from UP
+  double dt[8];
+  DevBlock B;
+};
+
 template <int NEQ, bool MHD>
-__global__ void __launch_bounds__(256, 4) viscous_kernel(ViscParams P) {
-  __shared__ DevBlock B;
-  __shared__ double pl[NEQ][18 * 18];   // plane k of W with the one-deep ghost frame from UP
-  const int t = threadIdx.x;
-  const int i = (t & 15) + 1, j = (t >> 4) + 1;
+__global__ void __launch_bounds__(STAGE_THREADS, NEQ <= 6 ? 3 : 2) viscous_kernel(ViscParams P) {
+  extern __shared__ __align__(16) unsigned char smraw[];
+  ViscSmem<NEQ>& S = *reinterpret_cast<ViscSmem<NEQ>*>(smraw);
+  DevBlock& B = S.B;
+  const int t = threadIdx.x, lane = t & (NC - 1);
+  const int slot = P.work[blockIdx.x / P.zsplit];
+  const int planes = NC / P.zsplit, z0 = 1 + (blockIdx.x % P.zsplit) * planes, z1 = z0 + planes - 1;
   const double eta = P.ph.eta;
-  Cfl<NEQ, MHD> cfl;
+  if (t < (int)(sizeof(DevBlock) / 4)) reinterpret_cast<int*>(&B)[t] = reinterpret_cast<const int*>(P.blocks + slot)[t];
+  __syncthreads();
   unsigned nonfinite = 0;
-  auto q = [](int ii, int jj) { return ii + 18 * jj; };
-  for (int w = blockIdx.x; w < P.nwork; w += gridDim.x) {
-    const int slot = P.work[w];
-    __syncthreads();
-    if (t < (int)(sizeof(DevBlock) / 4)) reinterpret_cast<int*>(&B)[t] = reinterpret_cast<const int*>(P.blocks + slot)[t];
-    __syncthreads();
-    cfl.block(B);
-    double wm[NEQ], wc[NEQ], wp[NEQ];
-    // W(k-1) for k=1 is the bottom ghost of UP
-    if (P.zero_ghost) {
+  if (t < PLANE) {
+    const int i = lane + 1, j = (t >> 4) + 1, h = i + (NC + 2) * j;
+    double* d0 = &S.pl[0][0][h];
+    double* w0 = P.w + cell_off(slot, NEQ, 0, i, j, 1);
+    auto fetch = [&](int k) {
+      double* d = d0 + (k & (VRING - 1)) * (NEQ * VPLANE);
+      const double* g = w0 + (k - 1) * PLANE;
 #pragma unroll
-      for (int e = 0; e < NEQ; ++e) wm[e] = 0.0;
-    } else {
-      gather_ghost<NEQ>(P.up, B, slot, i, j, 0, wm);
-    }
-    load_cell_rw<NEQ>(P.w, slot, i, j, 1, wc);
-    for (int k = 1; k <= NC; ++k) {
-      if (k < NC) load_cell_rw<NEQ>(P.w, slot, i, j, k + 1, wp);
-      else if (P.zero_ghost) {
+      for (int e = 0; e < NEQ; ++e) copy_async8(d + e * VPLANE, g + (size_t)e * BCELLS);
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // the column's cells below and above the slab
+    auto outside = [&](int k, double* u) {
+      if (k >= 1 && k <= NC) {
+        load_cell_rw<NEQ>(P.w, slot, i, j, k, u);
+      } else if (P.zero_ghost) {
 #pragma unroll
-        for (int e = 0; e < NEQ; ++e) wp[e] = 0.0;
+        for (int e = 0; e < NEQ; ++e) u[e] = 0.0;
       } else {
-        gather_ghost<NEQ>(P.up, B, slot, i, j, NC + 1, wp);
+        gather_ghost<NEQ>(P.up, B, slot, i, j, k, u);
       }
-      __syncthreads();
-#pragma unroll
-      for (int e = 0; e < NEQ; ++e) pl[e][q(i, j)] = wc[e];
-      if (t < 64) {  // one-deep x/y ghost frame of plane k from UP
-        const int side = t >> 4, r = (t & 15) + 1;
-        int gi, gj;
-        if (side == 0) { gi = 0; gj = r; }
-        else if (side == 1) { gi = NC + 1; gj = r; }
-        else if (side == 2) { gi = r; gj = 0; }
-        else { gi = r; gj = NC + 1; }
-        double g[NEQ];
-        if (P.zero_ghost) {
-#pragma unroll
-          for (int e = 0; e < NEQ; ++e) g[e] = 0.0;
-        } else {
-          gather_ghost<NEQ>(P.up, B, slot, gi, gj, k, g);
-        }
-#pragma unroll
-        for (int e = 0; e < NEQ; ++e) pl[e][q(gi, gj)] = g[e];
-      }
-      __syncthreads();
+    };
+    // one group per plane, empty past the slab, so the group counts match
+    for (int k = z0; k < z0 + 3; ++k) {
+      if (k <= z1) fetch(k);
+      else asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    double wm[NEQ], wt[NEQ];
+    outside(z0 - 1, wm);
+    outside(z1 + 1, wt);
+    Cfl<NEQ, MHD> cfl;
+    cfl.block(B);
+    if (P.zsplit > 1) cluster_barrier();
+    for (int k = z0; k <= z1; ++k) {
+      asm volatile("cp.async.wait_group 1;" ::: "memory");   // planes up to k+1
+      plane_barrier();
+      if (k + 3 <= z1) fetch(k + 3);                          // over plane k-1
+      else asm volatile("cp.async.commit_group;" ::: "memory");
+      const double* p = d0 + (k & (VRING - 1)) * (NEQ * VPLANE);
+      const double* pn = d0 + ((k + 1) & (VRING - 1)) * (NEQ * VPLANE);
       double un[NEQ];
+      double* o = w0 + (k - 1) * PLANE;
 #pragma unroll
       for (int e = 0; e < NEQ; ++e) {
-        const double c = wc[e];
-        un[e] = c + eta * (+pl[e][q(i + 1, j)] + pl[e][q(i - 1, j)] + pl[e][q(i, j + 1)] + pl[e][q(i, j - 1)] + wp[e] +
-                           wm[e] - 6.0 * c);
-      }
-      const size_t o = cell_off(slot, NEQ, 0, i, j, k);
-#pragma unroll
-      for (int e = 0; e < NEQ; ++e) {
-        P.w[o + (size_t)e * BCELLS] = un[e];
+        const double* q = p + e * VPLANE;
+        const double c = q[0], up = k < z1 ? pn[e * VPLANE] : wt[e];
+        un[e] = c + eta * (+q[1] + q[-1] + q[NC + 2] + q[-(NC + 2)] + up + wm[e] - 6.0 * c);
+        wm[e] = c;
+        o[(size_t)e * BCELLS] = un[e];
         nonfinite += !isfinite(un[e]);
       }
       if (P.do_dt) {
-        double p[NEQ], rinv;
-        flow2prim<NEQ, MHD>(un, p, P.ph.inv_cv, &rinv);
-        cfl.fold(p, rinv, B, P.ph.gamma);
+        double v[NEQ], rinv;
+        flow2prim<NEQ, MHD>(un, v, P.ph.inv_cv, &rinv);
+        cfl.fold(v, rinv, B, P.ph.gamma);
       }
+    }
+    if (P.do_dt) {
+      double v = cfl.dt();
+      for (int s = 16; s > 0; s >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, s));
+      if ((t & 31) == 0) S.dt[t >> 5] = v;
+    }
+    nonfinite = __reduce_add_sync(0xffffffffu, nonfinite);
+    if ((t & 31) == 0 && nonfinite) atomicAdd(&P.ctl->cnt[3], (unsigned long long)nonfinite);
+  } else {  // the frame cell of one (side, row) from UP
+    const int side = (t - PLANE) >> 4;
+    const int gi = side == 0 ? 0 : (side == 1 ? NC + 1 : lane + 1);
+    const int gj = side == 2 ? 0 : (side == 3 ? NC + 1 : lane + 1);
+    double* d0 = &S.pl[0][0][gi + (NC + 2) * gj];
+    double u[NEQ];
+    auto take = [&](int k) {
+      if (P.zero_ghost) {
 #pragma unroll
-      for (int e = 0; e < NEQ; ++e) { wm[e] = wc[e]; wc[e] = wp[e]; }
+        for (int e = 0; e < NEQ; ++e) u[e] = 0.0;
+      } else {
+        gather_ghost<NEQ>(P.up, B, slot, gi, gj, k, u);
+      }
+    };
+    take(z0);
+    if (P.zsplit > 1) cluster_barrier();
+    for (int k = z0; k <= z1; ++k) {
+      double* d = d0 + (k & (VRING - 1)) * (NEQ * VPLANE);
+#pragma unroll
+      for (int e = 0; e < NEQ; ++e) d[e * VPLANE] = u[e];
+      if (k < z1) take(k + 1);
+      plane_barrier();
     }
   }
-  if (P.do_dt) block_min_dt(cfl.dt(), P.ctl);
-  nonfinite = __reduce_add_sync(0xffffffffu, nonfinite);
-  if ((t & 31) == 0 && nonfinite) atomicAdd(&P.ctl->cnt[3], (unsigned long long)nonfinite);
+  if (P.do_dt) {
+    __syncthreads();
+    if (t == 0) {
+      double v = S.dt[0];
+      for (int k = 1; k < 8; ++k) v = fmin(v, S.dt[k]);
+      atomic_min_pos(&P.ctl->dtmin_bits, v);
+    }
+  }
 }
 
 // CFL minimum of an arbitrary state (getTimestep's loop, hydro_solver.f90:150-182).
@@ -1281,18 +1331,23 @@ struct DtParams {
   PhysParams ph;
 };
 
+// Items of two planes, so that a mesh of a few blocks still spreads over the
+// SMs (8 blocks: 10 -> 4 us).
+constexpr int DT_PLANES = 2;
 template <int NEQ, bool MHD>
 __global__ void __launch_bounds__(256) dt_kernel(DtParams P) {
   const int t = threadIdx.x;
   Cfl<NEQ, MHD> cfl;
-  for (int w = blockIdx.x; w < P.nwork; w += gridDim.x) {
-    const int slot = P.work[w];
+  for (int w = blockIdx.x; w < P.nwork * (NC / DT_PLANES); w += gridDim.x) {
+    const int slot = P.work[w / (NC / DT_PLANES)], k0 = w % (NC / DT_PLANES) * DT_PLANES;
     const DevBlock& B = P.blocks[slot];
+    double u[DT_PLANES][NEQ], p[NEQ], rinv;
+#pragma unroll
+    for (int k = 0; k < DT_PLANES; ++k) load_cell<NEQ>(P.u, slot, (t & 15) + 1, (t >> 4) + 1, k0 + k + 1, u[k]);
     cfl.block(B);
-    for (int k = 1; k <= NC; ++k) {
-      double u[NEQ], p[NEQ], rinv;
-      load_cell<NEQ>(P.u, slot, (t & 15) + 1, (t >> 4) + 1, k, u);
-      flow2prim<NEQ, MHD>(u, p, P.ph.inv_cv, &rinv);
+#pragma unroll
+    for (int k = 0; k < DT_PLANES; ++k) {
+      flow2prim<NEQ, MHD>(u[k], p, P.ph.inv_cv, &rinv);
       cfl.fold(p, rinv, B, P.ph.gamma);
     }
   }
@@ -1319,6 +1374,7 @@ __global__ void step_begin_kernel(DevCtl* ctl, double cfl, int cooling_on, doubl
     ctl->dumpout = 1;
   }
   ctl->dt = dt_glob;
+  ctl->work_next[0] = ctl->work_next[1] = 0;
   ctl->dtmin_bits = (unsigned long long)__double_as_longlong(1.0e30);
 }
 
