@@ -123,9 +123,9 @@ bool select_kern(const wx_config& c, Kern& k) {
   }
   if (c.neqtot != 8) return false;
   switch (rs) {
-    case WX_SOLVER_HLL: k = make_kern<8, true, WX_SOLVER_HLL, LIM_RUNTIME>(); return true;
-    case WX_SOLVER_HLLE: k = make_kern<8, true, WX_SOLVER_HLLE, LIM_RUNTIME>(); return true;
-    case WX_SOLVER_HLLD: k = make_kern<8, true, WX_SOLVER_HLLD, LIM_RUNTIME>(); return true;
+    case WX_SOLVER_HLL: k = make_kern_lim<8, true, WX_SOLVER_HLL>(lim); return true;
+    case WX_SOLVER_HLLE: k = make_kern_lim<8, true, WX_SOLVER_HLLE>(lim); return true;
+    case WX_SOLVER_HLLD: k = make_kern_lim<8, true, WX_SOLVER_HLLD>(lim); return true;
     default: return false;
   }
 }

@@ -123,6 +123,10 @@ __device__ __forceinline__ double mul_rsqrt_nr(double s, double x) {
   return fma(c * e, fma(0.375, e, 0.5), c);
 }
 __device__ __forceinline__ double sqrt_nr(double x) { return mul_rsqrt_nr(x, x); }
+// The same for the discriminant of the fast speeds, which may vanish, or fall
+// below zero by rounding (c_s = c_A along the field): zero there, the
+// library's root for the rest (subnormal, NaN).
+__device__ __forceinline__ double sqrt_nn(double x) { return x > 1.0e-290 ? sqrt_nr(x) : (x <= 0.0 ? 0.0 : sqrt(x)); }
 // Sound speed sqrt(gp / rho), gp = gamma p, as gp / sqrt(gp rho): one
 // estimate and no reciprocal of rho.
 __device__ __forceinline__ double sound_nr(double gp, double rho) { return mul_rsqrt_nr(gp, gp * rho); }
@@ -202,9 +206,9 @@ __device__ __forceinline__ void xflux(const double* p, double* f, double cv) {
 // cfastX (hydro_core.f90:553-566)
 __device__ __forceinline__ double cfastX(const double* p, double g) {
   const double b2 = p[5] * p[5] + p[6] * p[6] + p[7] * p[7];
-  const double rinv = 1.0 / p[0];
+  const double rinv = rcp_nr(p[0]);
   const double a = (g * p[4] + b2) * rinv;
-  return sqrt(0.5 * (a + sqrt(a * a - 4. * g * p[4] * (p[5] * p[5]) * rinv * rinv)));
+  return sqrt_nr(0.5 * (a + sqrt_nn(a * a - 4. * g * p[4] * (p[5] * p[5]) * rinv * rinv)));
 }
 
 // average (hydro_core.f90:640-699)
@@ -339,21 +343,22 @@ __device__ __forceinline__ void riemann_hllc_c(const double* pL, const double* p
   for (int e = 5; e < NEQ; ++e) f[e] = g * pk[e];
 }
 
-// HLL (hll.f90:175-260): Davis wave speeds, branches sl>=0 / sr<=0.
-template <int NEQ, bool MHD>
-__device__ __forceinline__ void riemann_hll(const double* pL, const double* pR, double* f, double g, double cv) {
-  const double cl = sqrt(g * pL[4] / pL[0]);
-  const double cr = sqrt(g * pR[4] / pR[0]);
+// HLL of MHD states (hll.f90:175-260): Davis wave speeds of the sound speed,
+// branches sl>=0 / sr<=0.
+template <int NEQ>
+__device__ __forceinline__ void riemann_hll_mhd(const double* pL, const double* pR, double* f, double g, double cv) {
+  const double cl = sound_nr(g * pL[4], pL[0]);
+  const double cr = sound_nr(g * pR[4], pR[0]);
   const double sl = dmin(pL[1] - cl, pR[1] - cr);
   const double sr = dmax(pL[1] + cl, pR[1] + cr);
-  if (sl >= 0.0) { xflux<NEQ, MHD>(pL, f, cv); return; }
-  if (sr <= 0.0) { xflux<NEQ, MHD>(pR, f, cv); return; }
+  if (sl >= 0.0) { xflux<NEQ, true>(pL, f, cv); return; }
+  if (sr <= 0.0) { xflux<NEQ, true>(pR, f, cv); return; }
   double fL[NEQ], fR[NEQ], uL[NEQ], uR[NEQ];
-  xflux<NEQ, MHD>(pL, fL, cv);
-  xflux<NEQ, MHD>(pR, fR, cv);
-  prim2flow<NEQ, MHD>(pL, uL, cv);
-  prim2flow<NEQ, MHD>(pR, uR, cv);
-  const double inv = 1.0 / (sr - sl);
+  xflux<NEQ, true>(pL, fL, cv);
+  xflux<NEQ, true>(pR, fR, cv);
+  prim2flow<NEQ, true>(pL, uL, cv);
+  prim2flow<NEQ, true>(pR, uR, cv);
+  const double inv = rcp_nr(sr - sl);
   const double slsr = sl * sr;
 #pragma unroll
   for (int e = 0; e < NEQ; ++e) f[e] = (sr * fL[e] - sl * fR[e] + slsr * (uR[e] - uL[e])) * inv;
@@ -372,7 +377,7 @@ __device__ __forceinline__ void riemann_hlle(const double* pL, const double* pR,
   xflux<NEQ, true>(pR, fR, cv);
   prim2flow<NEQ, true>(pL, uL, cv);
   prim2flow<NEQ, true>(pR, uR, cv);
-  const double inv = 1.0 / (sr - sl);
+  const double inv = rcp_nr(sr - sl);
   const double slsr = sl * sr;
 #pragma unroll
   for (int e = 0; e < NEQ; ++e) f[e] = (sr * fL[e] - sl * fR[e] + slsr * (uR[e] - uL[e])) * inv;
@@ -397,15 +402,17 @@ __device__ __forceinline__ void riemann_hlld(const double* pl, const double* pr,
   const double slmul = sl - pl[1];
   const double srmur = sr - pr[1];
   const double den = srmur * pr[0] - slmul * pl[0];
-  const double sM = (srmur * (pr[0] * pr[1]) - slmul * (pl[0] * pl[1]) - pTR + pTL) / den;
+  const double rden = rcp_nr(den);
+  const double sM = (srmur * (pr[0] * pr[1]) - slmul * (pl[0] * pl[1]) - pTR + pTL) * rden;
   const double srmsM = sr - sM;
   const double slmsM = sl - sM;
-  const double rhostl = pl[0] * slmul / slmsM;
-  const double rhostr = pr[0] * srmur / srmsM;
-  const double sqrl = sqrt(rhostl), sqrr = sqrt(rhostr);
-  const double sstl = sM - fabs(bx) / sqrl;
-  const double sstr = sM + fabs(bx) / sqrr;
-  const double pst = (srmur * pr[0] * pTL - slmul * pl[0] * pTR + pl[0] * pr[0] * srmur * slmul * (pr[1] - pl[1])) / den;
+  const double rsl = rcp_nr(slmsM), rsr = rcp_nr(srmsM);
+  const double rhostl = pl[0] * slmul * rsl;
+  const double rhostr = pr[0] * srmur * rsr;
+  const double sqrl = sqrt_nr(rhostl), sqrr = sqrt_nr(rhostr);
+  const double sstl = sM - mul_rsqrt_nr(fabs(bx), rhostl);
+  const double sstr = sM + mul_rsqrt_nr(fabs(bx), rhostr);
+  const double pst = (srmur * pr[0] * pTL - slmul * pl[0] * pTR + pl[0] * pr[0] * srmur * slmul * (pr[1] - pl[1])) * rden;
   const bool leftside = (sstl >= 0.0) || (!(sstr <= 0.0) && (sM >= 0.0));
   // star state of the left or right side
   double vstl = 0, wstl = 0, bystl = 0, bzstl = 0, vstr = 0, wstr = 0, bystr = 0, bzstr = 0;
@@ -417,7 +424,7 @@ __device__ __forceinline__ void riemann_hlld(const double* pl, const double* pr,
   if (needL) {
     if (denl == 0) { vstl = pl[2]; wstl = pl[3]; bystl = 0.; bzstl = 0.; }
     else {
-      const double q = 1.0 / denl;
+      const double q = rcp_nr(denl);
       vstl = pl[2] - bx * pl[6] * sMmul * q;
       wstl = pl[3] - bx * pl[7] * sMmul * q;
       const double t = (pl[0] * (slmul * slmul) - bx2) * q;
@@ -430,7 +437,7 @@ __device__ __forceinline__ void riemann_hlld(const double* pl, const double* pr,
       if (sstr <= 0.0) { vstl = pl[2]; wstl = pl[3]; bystl = 0.; bzstl = 0.; }
       else { vstr = pr[2]; wstr = pr[3]; bystr = 0.; bzstr = 0.; }
     } else {
-      const double q = 1.0 / denr;
+      const double q = rcp_nr(denr);
       vstr = pr[2] - bx * pr[6] * sMmur * q;
       wstr = pr[3] - bx * pr[7] * sMmur * q;
       const double t = (pr[0] * (srmur * srmur) - bx2) * q;
@@ -440,7 +447,7 @@ __device__ __forceinline__ void riemann_hlld(const double* pl, const double* pr,
   }
   const double* pk = leftside ? pl : pr;
   const double skmu = leftside ? slmul : srmur;
-  const double skms = leftside ? slmsM : srmsM;
+  const double rsk = leftside ? rsl : rsr;
   const double pTk = leftside ? pTL : pTR;
   const double rhost = leftside ? rhostl : rhostr;
   const double ek = 0.5 * pk[0] * (pk[1] * pk[1] + pk[2] * pk[2] + pk[3] * pk[3]) + cv * pk[4] +
@@ -449,7 +456,7 @@ __device__ __forceinline__ void riemann_hlld(const double* pl, const double* pr,
   const double vst = leftside ? vstl : vstr, wst = leftside ? wstl : wstr;
   const double byst = leftside ? bystl : bystr, bzst = leftside ? bzstl : bzstr;
   const double vstdotbst = sM * bx + vst * byst + wst * bzst;
-  const double est = (skmu * ek - pTk * pk[1] + pst * sM + bx * (vdotb - vstdotbst)) / skms;
+  const double est = (skmu * ek - pTk * pk[1] + pst * sM + bx * (vdotb - vstdotbst)) * rsk;
   if ((sstl >= 0.0) || (sstr <= 0.0)) {  // UL* or UR*
     ff[0] = rhost * sM;
     ff[1] = rhost * (sM * sM) + pst - bx2;
@@ -462,10 +469,10 @@ __device__ __forceinline__ void riemann_hlld(const double* pl, const double* pr,
     return;
   }
   const double dd = sqrl + sqrr;
-  const double ddi = 1.0 / dd;
+  const double ddi = rcp_nr(dd);
   const double vstst = (sqrl * vstl + sqrr * vstr + (bystr - bystl) * signBx) * ddi;
   const double wstst = (sqrl * wstl + sqrr * wstr + (bzstr - bzstl) * signBx) * ddi;
-  const double sqlr = sqrt(rhostl * rhostr);
+  const double sqlr = sqrl * sqrr;
   const double bystst = (sqrl * bystr + sqrr * bystl + sqlr * (vstr - vstl) * signBx) * ddi;
   const double bzstst = (sqrl * bzstr + sqrr * bzstl + sqlr * (wstr - wstl) * signBx) * ddi;
   const double vststdotbstst = sM * bx + vstst * bystst + wstst * bzstst;
@@ -487,7 +494,7 @@ template <int NEQ, int SOLVER>
 __device__ __forceinline__ void riemann_mhd(const double* pL, const double* pR, double* f, double g, double cv) {
   if constexpr (SOLVER == WX_SOLVER_HLLE) riemann_hlle<NEQ>(pL, pR, f, g, cv);
   else if constexpr (SOLVER == WX_SOLVER_HLLD) riemann_hlld<NEQ>(pL, pR, f, g, cv);
-  else riemann_hll<NEQ, true>(pL, pR, f, g, cv);
+  else riemann_hll_mhd<NEQ>(pL, pR, f, g, cv);
 }
 
 // ---------------------------------------------------------------------------
@@ -587,53 +594,42 @@ __device__ __forceinline__ void get_cell(const double* __restrict__ a, const Dev
   else gather_ghost<NEQ>(a, b, slot, i, j, k, u);
 }
 
-// CFL time step of one cell (hydro_core.f90:503-543, hydro_solver.f90:441-455).
-template <int NEQ, bool MHD>
-__device__ __forceinline__ double cell_dt(const double* p, const DevBlock& B, double g) {
-  if (MHD) {
-    const double b2 = p[5] * p[5] + p[6] * p[6] + p[7] * p[7];
-    const double a = g * p[4] + b2;
-    const double cfx = sqrt(0.5 * (a + sqrt(a * a - 4. * g * p[4] * p[5] * p[5])) / p[0]);
-    const double cfy = sqrt(0.5 * (a + sqrt(a * a - 4. * g * p[4] * p[6] * p[6])) / p[0]);
-    const double cfz = sqrt(0.5 * (a + sqrt(a * a - 4. * g * p[4] * p[7] * p[7])) / p[0]);
-    return dmin(dmin(B.dx / (fabs(p[1]) + cfx), B.dy / (fabs(p[2]) + cfy)), B.dz / (fabs(p[3]) + cfz));
-  }
-  const double cs = sqrt(g * p[4] / p[0]);
-  return dmin(dmin(B.dx / (fabs(p[1]) + cs), B.dy / (fabs(p[2]) + cs)), B.dz / (fabs(p[3]) + cs));
-}
-
-// The CFL condition of a hydro cell as a signal speed over the cell size,
-// max_d (|u_d| + c)/dx_d, whose reciprocal is cell_dt's
-// min_d dx_d/(|u_d| + c).  A block's kernels keep the largest speed and take
-// one reciprocal at the end, so the per-cell work has no division.  idx..idz
-// are 1/dx..1/dz; rinv is 1/rho of flow2prim.
+// The CFL condition of a cell (hydro_core.f90:503-543,
+// hydro_solver.f90:441-455) as a signal speed over the cell size,
+// max_d (|u_d| + c_d)/dx_d, whose reciprocal is the reference's
+// min_d dx_d/(|u_d| + c_d); c_d is the sound speed, or for MHD the fast speed
+// along d.  The kernels keep the largest speed and take one reciprocal at the
+// end, so the per-cell work has no division.  idx..idz are 1/dx..1/dz; rinv
+// is 1/rho of flow2prim.
+template <bool MHD>
 __device__ __forceinline__ double cell_cfl_speed(const double* p, double rinv, double idx, double idy, double idz,
                                                  double g) {
+  if constexpr (MHD) {
+    const double a = g * p[4] + (p[5] * p[5] + p[6] * p[6] + p[7] * p[7]);
+    const double q = 4. * g * p[4];
+    const double cfx = sqrt_nr(0.5 * (a + sqrt_nn(a * a - q * p[5] * p[5])) * rinv);
+    const double cfy = sqrt_nr(0.5 * (a + sqrt_nn(a * a - q * p[6] * p[6])) * rinv);
+    const double cfz = sqrt_nr(0.5 * (a + sqrt_nn(a * a - q * p[7] * p[7])) * rinv);
+    return dmax(dmax((fabs(p[1]) + cfx) * idx, (fabs(p[2]) + cfy) * idy), (fabs(p[3]) + cfz) * idz);
+  }
   const double cs = sqrt_nr(g * p[4] * rinv);
   return dmax(dmax((fabs(p[1]) + cs) * idx, (fabs(p[2]) + cs) * idy), (fabs(p[3]) + cs) * idz);
 }
 
-// One thread's running CFL reduction over the cells it visits: for hydro the
-// largest cell_cfl_speed (one reciprocal at the end), for MHD the smallest
-// cell_dt.  block() takes the inverse cell sizes of the block being walked.
+// One thread's running CFL reduction over the cells it visits.  block() takes
+// the inverse cell sizes of the block being walked.
 template <int NEQ, bool MHD>
 struct Cfl {
-  double acc = MHD ? 1.0e300 : 0.0;
+  double acc = 0.0;
   double idx = 0.0, idy = 0.0, idz = 0.0;
-  __device__ __forceinline__ void block(const DevBlock& B) {
-    if (!MHD) { idx = 1.0 / B.dx; idy = 1.0 / B.dy; idz = 1.0 / B.dz; }
-  }
-  __device__ __forceinline__ void fold(const double* p, double rinv, const DevBlock& B, double g) {
-    fold(p, rinv, B, idx, idy, idz, g);
-  }
+  __device__ __forceinline__ void block(const DevBlock& B) { idx = 1.0 / B.dx; idy = 1.0 / B.dy; idz = 1.0 / B.dz; }
+  __device__ __forceinline__ void fold(const double* p, double rinv, double g) { fold(p, rinv, idx, idy, idz, g); }
   // the same with the inverse cell sizes passed in (block() not used)
-  __device__ __forceinline__ void fold(const double* p, double rinv, const DevBlock& B, double ix, double iy,
-                                       double iz, double g) {
-    if constexpr (MHD) acc = dmin(acc, cell_dt<NEQ, MHD>(p, B, g));
-    else acc = dmax(acc, cell_cfl_speed(p, rinv, ix, iy, iz, g));
+  __device__ __forceinline__ void fold(const double* p, double rinv, double ix, double iy, double iz, double g) {
+    acc = dmax(acc, cell_cfl_speed<MHD>(p, rinv, ix, iy, iz, g));
   }
   // the thread's time step (infinite when it saw no cell)
-  __device__ __forceinline__ double dt() const { return MHD ? acc : 1.0 / acc; }
+  __device__ __forceinline__ double dt() const { return 1.0 / acc; }
 };
 
 // Ordered bit patterns of positive doubles compare like the doubles.

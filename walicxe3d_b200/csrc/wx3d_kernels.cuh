@@ -167,7 +167,7 @@ __device__ __forceinline__ void iface_flux(const double* c0, const double* c1, c
 // Stores the result of the fused viscous step for one cell, counts
 // non-finite values and folds the cell's CFL time step.
 template <int NEQ, bool MHD>
-__device__ __forceinline__ void visc_store(const StageParams& P, const DevBlock& B, const double* un, size_t o,
+__device__ __forceinline__ void visc_store(const StageParams& P, const double* un, size_t o,
                                            Cfl<NEQ, MHD>& cfl, StageConsts& K) {
   unsigned nonfinite = 0;
 #pragma unroll
@@ -179,7 +179,7 @@ __device__ __forceinline__ void visc_store(const StageParams& P, const DevBlock&
   if (P.do_dt) {
     double p[NEQ], rinv;
     flow2prim<NEQ, MHD>(un, p, P.ph.inv_cv, &rinv);
-    cfl.fold(p, rinv, B, K.idx, K.idy, K.idz, P.ph.gamma);
+    cfl.fold(p, rinv, K.idx, K.idy, K.idz, P.ph.gamma);
   }
 }
 
@@ -245,7 +245,11 @@ __device__ __forceinline__ void load_plane(const StageParams& P, const DevBlock&
 // neighbours - 6 W) to plane m-1, whose z-neighbours are W(m-2) (still in
 // the buffer slot that W(m) replaces, read first by the same thread) and
 // W(m) (in registers).  The block-face z-neighbours are UP ghosts as well.
-// One CTA per SM (168 registers, 105-200 KB of shared memory).
+// One CTA per SM (168 registers, 105-200 KB of shared memory): bound by the
+// FP64 chains of HLLD.  Refined reciprocals and roots in place of its nine
+// divisions and seven roots per interface, and minmod compiled in as for
+// hydro: 440 blocks (HLLD) predictor 0.394 -> 0.270 ms, corrector with the
+// viscous step 0.912 -> 0.430 ms; 16 blocks in 8 slabs 29 + 50 -> 20 + 24 us.
 
 // Cell-centred electric field E = -v x B of the stage primitives at one ring
 // cell: the field-interpolated E of the field-CD scheme (Toth 2000, J. Comput.
@@ -406,9 +410,9 @@ __global__ void __launch_bounds__(STAGE_THREADS, 1) stage_kernel(StageParams P) 
           const double* pm = ring + ring_slot(m) * NEQ * Geo<ORDER>::PL;
           const double* pu = ring + ring_slot(m + 1) * NEQ * Geo<ORDER>::PL;
           const int h = hc;
-          const double divB = (pm[5 * Geo<ORDER>::PL + h + 1] - pm[5 * Geo<ORDER>::PL + h - 1]) / (2. * B.dx) +
-                              (pm[6 * Geo<ORDER>::PL + h + Geo<ORDER>::W] - pm[6 * Geo<ORDER>::PL + h - Geo<ORDER>::W]) / (2. * B.dy) +
-                              (pu[7 * Geo<ORDER>::PL + h] - bz_below) / (2. * B.dz);
+          const double divB = (pm[5 * Geo<ORDER>::PL + h + 1] - pm[5 * Geo<ORDER>::PL + h - 1]) * (0.5 * K.idx) +
+                              (pm[6 * Geo<ORDER>::PL + h + Geo<ORDER>::W] - pm[6 * Geo<ORDER>::PL + h - Geo<ORDER>::W]) * (0.5 * K.idy) +
+                              (pu[7 * Geo<ORDER>::PL + h] - bz_below) * (0.5 * K.idz);
           const double v1 = pm[1 * Geo<ORDER>::PL + h], v2 = pm[2 * Geo<ORDER>::PL + h], v3 = pm[3 * Geo<ORDER>::PL + h];
           const double b1 = pm[5 * Geo<ORDER>::PL + h], b2 = pm[6 * Geo<ORDER>::PL + h], b3 = pm[7 * Geo<ORDER>::PL + h];
           s[1] = -divB * b1;
@@ -466,7 +470,7 @@ __global__ void __launch_bounds__(STAGE_THREADS, 1) stage_kernel(StageParams P) 
               un[e] = c + ph.eta * (+pe[vq(ci + 1, cj)] + pe[vq(ci - 1, cj)] + pe[vq(ci, cj + 1)] + pe[vq(ci, cj - 1)] +
                                     wv[e] + wb[e * VPLANE + vq(ci, cj)] - 6.0 * c);
             }
-            visc_store<NEQ, true>(P, B, un, o - NC * NC, cfl, K);
+            visc_store<NEQ, true>(P, un, o - NC * NC, cfl, K);
           }
 #pragma unroll
           for (int e = 0; e < NEQ; ++e) wb[e * VPLANE + vq(ci, cj)] = wv[e];
@@ -488,7 +492,7 @@ __global__ void __launch_bounds__(STAGE_THREADS, 1) stage_kernel(StageParams P) 
         un[e] = c + ph.eta * (+pe[vq(ci + 1, cj)] + pe[vq(ci - 1, cj)] + pe[vq(ci, cj + 1)] + pe[vq(ci, cj - 1)] + g[e] +
                               wb[e * VPLANE + vq(ci, cj)] - 6.0 * c);
       }
-      visc_store<NEQ, true>(P, B, un, cell_off(slot, NEQ, 0, ci, cj, z1), cfl, K);
+      visc_store<NEQ, true>(P, un, cell_off(slot, NEQ, 0, ci, cj, z1), cfl, K);
     }
     // items past the first wave go, in list order, to whichever CTA
     // finishes first (the counter is zeroed before each launch): blocks at
@@ -1033,7 +1037,7 @@ __global__ void __launch_bounds__(STAGE_THREADS, (corr_ctas_per_sm<NEQ, VISC>())
             S.w[b][e][h] = v[e];
             v[e] = pw[0] + ph.eta * ((pw[1] + pw[-1]) + (pw[W] + pw[-W]) + (v[e] + below) - 6.0 * pw[0]);
           }
-          if (m > z0) visc_store<NEQ, false>(P, B, v, o - NC * NC, cfl, K);
+          if (m > z0) visc_store<NEQ, false>(P, v, o - NC * NC, cfl, K);
         }
         if (m < z1) fetch(m + 3);  // over plane m, which no one reads any more
       }
@@ -1046,7 +1050,7 @@ __global__ void __launch_bounds__(STAGE_THREADS, (corr_ctas_per_sm<NEQ, VISC>())
           const double* pw = &S.w[z1 & 1][e][h];
           un[e] = pw[0] + ph.eta * ((pw[1] + pw[-1]) + (pw[W] + pw[-W]) + (g[e] + S.w[(z1 - 1) & 1][e][h]) - 6.0 * pw[0]);
         }
-        visc_store<NEQ, false>(P, B, un, cell_off(slot, NEQ, 0, ci, cj, z1), cfl, K);
+        visc_store<NEQ, false>(P, un, cell_off(slot, NEQ, 0, ci, cj, z1), cfl, K);
       }
     } else {
       double g2[NEQ];  // primitives of the outer ghost; the inner one's are in the frame
@@ -1277,7 +1281,7 @@ __global__ void __launch_bounds__(STAGE_THREADS, NEQ <= 6 ? 3 : 2) viscous_kerne
       if (P.do_dt) {
         double v[NEQ], rinv;
         flow2prim<NEQ, MHD>(un, v, P.ph.inv_cv, &rinv);
-        cfl.fold(v, rinv, B, P.ph.gamma);
+        cfl.fold(v, rinv, P.ph.gamma);
       }
     }
     if (P.do_dt) {
@@ -1348,7 +1352,7 @@ __global__ void __launch_bounds__(256) dt_kernel(DtParams P) {
 #pragma unroll
     for (int k = 0; k < DT_PLANES; ++k) {
       flow2prim<NEQ, MHD>(u[k], p, P.ph.inv_cv, &rinv);
-      cfl.fold(p, rinv, B, P.ph.gamma);
+      cfl.fold(p, rinv, P.ph.gamma);
     }
   }
   block_min_dt(cfl.dt(), P.ctl);

@@ -783,7 +783,7 @@ __device__ __forceinline__ void fallback_cell(const SurrParams& P, int id, doubl
   P.u[o + 5 * (size_t)BCELLS] = u[5];
   if (P.do_dt) {
     const DevBlock& B = P.blocks[slot];
-    cfl.fold(p, rinv, B, 1.0 / B.dx, 1.0 / B.dy, 1.0 / B.dz, ph.gamma);
+    cfl.fold(p, rinv, 1.0 / B.dx, 1.0 / B.dy, 1.0 / B.dz, ph.gamma);
   }
 }
 
@@ -875,7 +875,7 @@ __global__ void __launch_bounds__(TILE, 4) surrogate_source_kernel(SurrParams P)
         P.u[o + 5 * (size_t)BCELLS] = p[5];
         if (P.do_dt) {
           const DevBlock& B = P.blocks[slot];
-          cfl.fold(p, rinv, B, 1.0 / B.dx, 1.0 / B.dy, 1.0 / B.dz, ph.gamma);
+          cfl.fold(p, rinv, 1.0 / B.dx, 1.0 / B.dy, 1.0 / B.dz, ph.gamma);
         }
         ++nsur;
       }

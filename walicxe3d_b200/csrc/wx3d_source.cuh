@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(256, 5) source_kernel(SrcParams P) {
         P.prim[o + 4 * (size_t)BCELLS] = p[4];
         if (HAS_PAS) P.prim[o + (size_t)fp * BCELLS] = p[fp];
       }
-      if (do_dt) cfl.fold(p, rinv, B, inv_dx[0], inv_dx[1], inv_dx[2], ph.gamma);
+      if (do_dt) cfl.fold(p, rinv, inv_dx[0], inv_dx[1], inv_dx[2], ph.gamma);
     }
   }
   if (do_dt) {
