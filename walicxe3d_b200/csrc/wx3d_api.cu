@@ -1775,14 +1775,33 @@ int wx3d_read_state(wx_ctx* c, const char* path, int32_t* noutput, char* datadir
   return WX_OK;
 }
 
+// The physical cells U(1:ns, :, 1:16, 1:16, kf) of a plane of the Fortran
+// array, to or from the staging slab [j][i][eq][nbmax], and nothing else: the
+// ghosts and the entries past ns neither travel nor change.  Where every
+// entry travels, a row of 16 cells is one contiguous run.
+static cudaError_t copy_fortran_plane(wx_ctx* c, int nbmax, int ns, int kf, double* U, bool up) {
+  double* h = U + (size_t)nbmax * c->neq * (400 * (size_t)(kf + 1) + 20 * 2 + 2);
+  const size_t cell = (size_t)nbmax * c->neq * 8;   // bytes of one cell's entries
+  cudaMemcpy3DParms p{};
+  const bool rows = ns == nbmax;
+  const cudaPitchedPtr host = rows ? make_cudaPitchedPtr(h, 20 * cell, 20 * cell, 20)
+                                   : make_cudaPitchedPtr(h, (size_t)nbmax * 8, (size_t)nbmax * 8, 20 * (size_t)c->neq);
+  const cudaPitchedPtr dev = rows ? make_cudaPitchedPtr(c->dStage, 16 * cell, 16 * cell, 16)
+                                  : make_cudaPitchedPtr(c->dStage, (size_t)nbmax * 8, (size_t)nbmax * 8, 16 * (size_t)c->neq);
+  p.srcPtr = up ? host : dev;
+  p.dstPtr = up ? dev : host;
+  p.extent = rows ? make_cudaExtent(16 * cell, 16, 1) : make_cudaExtent((size_t)ns * 8, 16 * (size_t)c->neq, 16);
+  p.kind = up ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
+  return cudaMemcpy3DAsync(&p, c->stream);
+}
+
 int wx3d_upload_U_fortran(wx_ctx* c, int32_t nbmax, const double* U) {
   if (!c || !U || nbmax <= 0) return WX_ERR_INVALID_ARG;
   const int ns = std::min(nbmax, c->max_blocks);
-  const size_t slab = (size_t)nbmax * c->neq * 400;  // U(:,:,:,:,k) for one k
   int rc;
-  if ((rc = ensure_stage(c, slab * 8))) return rc;
+  if ((rc = ensure_stage(c, (size_t)nbmax * c->neq * PLANE * 8))) return rc;
   for (int kf = 1; kf <= NC; ++kf) {
-    WX_CUDA(cudaMemcpyAsync(c->dStage, U + slab * (size_t)(kf + 1), slab * 8, cudaMemcpyHostToDevice, c->stream));
+    WX_CUDA(copy_fortran_plane(c, nbmax, ns, kf, const_cast<double*>(U), true));
     fortran_to_native<<<c->nsm * 4, 256, 0, c->stream>>>(c->dStage, c->dU, nbmax, ns, c->neq, kf);
     WX_LAUNCHED();
   }
@@ -1796,15 +1815,12 @@ int wx3d_upload_U_fortran(wx_ctx* c, int32_t nbmax, const double* U) {
 int wx3d_download_U_fortran(wx_ctx* c, int32_t nbmax, double* U) {
   if (!c || !U || nbmax <= 0) return WX_ERR_INVALID_ARG;
   const int ns = std::min(nbmax, c->max_blocks);
-  const size_t slab = (size_t)nbmax * c->neq * 400;
   int rc;
-  if ((rc = ensure_stage(c, slab * 8))) return rc;
+  if ((rc = ensure_stage(c, (size_t)nbmax * c->neq * PLANE * 8))) return rc;
   for (int kf = 1; kf <= NC; ++kf) {
-    // keep the ghost and unused entries of the caller's slab
-    WX_CUDA(cudaMemcpyAsync(c->dStage, U + slab * (size_t)(kf + 1), slab * 8, cudaMemcpyHostToDevice, c->stream));
     native_to_fortran<<<c->nsm * 4, 256, 0, c->stream>>>(c->dU, c->dStage, nbmax, ns, c->neq, kf);
     WX_LAUNCHED();
-    WX_CUDA(cudaMemcpyAsync(U + slab * (size_t)(kf + 1), c->dStage, slab * 8, cudaMemcpyDeviceToHost, c->stream));
+    WX_CUDA(copy_fortran_plane(c, nbmax, ns, kf, U, false));
   }
   WX_CUDA(cudaStreamSynchronize(c->stream));
   return WX_OK;
