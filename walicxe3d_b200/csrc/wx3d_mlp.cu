@@ -288,6 +288,7 @@ struct __align__(128) FwdSmem {
   __nv_bfloat16 h2[TILE * 128];   // [128][128] SiLU(z2), cols 64.. = (1, 0, ...)
   __nv_bfloat16 w[PK_N];          // packed weights
   float b1[NH], b2[NH], w3[NH * NOUT], b3[16];
+  float lsum[4];                  // loss of each warp
   uint64_t bar;
   uint32_t tmem;
   int err;
@@ -335,6 +336,31 @@ __device__ void load_weights(S& s, const __nv_bfloat16* __restrict__ pk, const f
   }
   for (int i = threadIdx.x; i < NH * NOUT; i += blockDim.x) s.w3[i] = prm[OFF_W3 + i];
   if (threadIdx.x < 16) s.b3[threadIdx.x] = threadIdx.x < NOUT ? prm[OFF_B3 + threadIdx.x] : 0.f;
+}
+
+// Gradient of one training CTA, as its TMEM rows deliver it: 64 columns of
+// dW2 and two of dW3, each of 65 rows (row 64: db2, db3), then five columns of
+// dW1^T of 64 rows (column 4: db1), then the CTA's loss.
+// PG_GROUPS such vectors are kept (0.3 MB); CTA b adds to vector b mod
+// PG_GROUPS, so at most ten CTAs meet in an element, 32 consecutive floats at
+// a time (the parameters' own order put every lane in another sector and all
+// CTAs in one element: 41 us a batch of 128 tiles against 26).
+constexpr int PG_GROUPS = 16;
+constexpr int PG_W3 = NH * (NH + 1), PG_W1 = PG_W3 + NOUT * (NH + 1), PG_LOSS = PG_W1 + (NIN + 1) * NH, PG_N = PG_LOSS + 1;
+static_assert(PG_LOSS == NPARAM, "one gradient element per parameter");
+
+// The parameter of gradient element q.
+__device__ __forceinline__ int pg_param(int q) {
+  if (q < PG_W3) {
+    const int c = q / (NH + 1), r = q % (NH + 1);
+    return r < NH ? OFF_W2 + r * NH + c : OFF_B2 + c;
+  }
+  if (q < PG_W1) {
+    const int c = (q - PG_W3) / (NH + 1), r = (q - PG_W3) % (NH + 1);
+    return r < NH ? OFF_W3 + r * NOUT + c : OFF_B3 + c;
+  }
+  const int c = (q - PG_W1) / NH, r = (q - PG_W1) % NH;
+  return c < NIN ? OFF_W1 + c * NH + r : OFF_B1 + r;
 }
 
 // Writes the padding columns 64..127 of an activation row: 1 at column 64.
@@ -501,8 +527,8 @@ __global__ void __launch_bounds__(TILE, 4) forward_kernel(const float* __restric
 __global__ void __launch_bounds__(TILE) train_kernel(const float* __restrict__ in, const float* __restrict__ tgt,
                                                       long long n, long long first_tile, int tiles, float gscale,
                                                       const __nv_bfloat16* __restrict__ pk,
-                                                      const float* __restrict__ prm, float* __restrict__ grad,
-                                                      float* __restrict__ loss, int* err) {
+                                                      const float* __restrict__ prm, float* __restrict__ part,
+                                                      int* err) {
   extern __shared__ __align__(128) unsigned char smraw[];
   FwdSmem& s = *reinterpret_cast<FwdSmem*>(smraw);
   BwdSmem& b = *reinterpret_cast<BwdSmem*>(smraw + ((sizeof(FwdSmem) + 127) / 128) * 128);
@@ -641,12 +667,14 @@ __global__ void __launch_bounds__(TILE) train_kernel(const float* __restrict__ i
     phase ^= 1;
     fence_after();
   }
-  // flush the accumulated weight gradients: lanes (= rows) 0..63 hold the
-  // hidden units, lane 64 the bias row.  The TMEM loads are warp-collective,
-  // so every thread issues them and only the owners of a row add it.
+  // the CTA's gradient and loss are added to its group's vector of `part`:
+  // lanes (= rows) 0..63 hold the hidden units, lane 64 the bias row.  The
+  // TMEM loads are warp-collective, so every thread issues them and only the
+  // owners of a row add it.
   ok = __syncthreads_and(ok);
   const int row = t;
   const long long first = first_tile + (long long)blockIdx.x * tiles;
+  float* pg = part + (blockIdx.x % PG_GROUPS) * PG_N;
   if (ok && first < ntiles) {
     float g[64], g3[16], g1[16];
 #pragma unroll
@@ -654,41 +682,27 @@ __global__ void __launch_bounds__(TILE) train_kernel(const float* __restrict__ i
     tmem_ld16(tmem_addr(tb, 256), g3);
     tmem_ld16(tmem_addr(tb, 352), g1);
     tmem_wait_ld();
+    if (row <= 64) {
+#pragma unroll
+      for (int c = 0; c < NH; ++c) atomicAdd(&pg[c * (NH + 1) + row], g[c]);
+#pragma unroll
+      for (int c = 0; c < NOUT; ++c) atomicAdd(&pg[PG_W3 + c * (NH + 1) + row], g3[c]);
+    }
     if (row < 64) {
-      // dW2: row = hidden1 unit j, columns = hidden2 units -> W2[j][.]
-      for (int i2 = 0; i2 < 64; ++i2) atomicAdd(&grad[OFF_W2 + row * NH + i2], g[i2]);
-      atomicAdd(&grad[OFF_W3 + row * NOUT + 0], g3[0]);
-      atomicAdd(&grad[OFF_W3 + row * NOUT + 1], g3[1]);
-      for (int i2 = 0; i2 < NIN; ++i2) atomicAdd(&grad[OFF_W1 + i2 * NH + row], g1[i2]);
-      atomicAdd(&grad[OFF_B1 + row], g1[4]);
-    } else if (row == 64) {
-      for (int i2 = 0; i2 < 64; ++i2) atomicAdd(&grad[OFF_B2 + i2], g[i2]);
-      atomicAdd(&grad[OFF_B3 + 0], g3[0]);
-      atomicAdd(&grad[OFF_B3 + 1], g3[1]);
+#pragma unroll
+      for (int c = 0; c <= NIN; ++c) atomicAdd(&pg[PG_W1 + c * NH + row], g1[c]);
     }
   }
-  // loss: warp reduce then one atomic per warp
   for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-  if ((t & 31) == 0 && loss) atomicAdd(loss, lsum * gscale);
+  if ((t & 31) == 0) s.lsum[t >> 5] = lsum;
+  __syncthreads();
+  if (t == 0) atomicAdd(&pg[PG_LOSS], (s.lsum[0] + s.lsum[1] + s.lsum[2] + s.lsum[3]) * gscale);
   if (!ok && t == 0) s.err = 1;
   fence_before();
   __syncthreads();
   fence_after();
   if (t < 32) tmem_free(s.tmem, 512);
   if (t == 0 && s.err) atomicAdd(err, 1);
-}
-
-// Adam on the FP32 master parameters, then repacks the bf16 operand images.
-__global__ void adam_kernel(float* __restrict__ prm, const float* __restrict__ grad, float* __restrict__ m,
-                            float* __restrict__ v, float lr, float b1, float b2, float eps, float c1, float c2) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < NPARAM; i += gridDim.x * blockDim.x) {
-    const float g = grad[i];
-    const float mi = b1 * m[i] + (1.f - b1) * g;
-    const float vi = b2 * v[i] + (1.f - b2) * g * g;
-    m[i] = mi;
-    v[i] = vi;
-    prm[i] -= lr * (mi * c1) / (sqrtf(vi * c2) + eps);
-  }
 }
 
 // Row and column of element o of a core-matrix image with C columns.
@@ -727,6 +741,67 @@ __global__ void pack_kernel(const float* __restrict__ prm, __nv_bfloat16* __rest
       v = prm[OFF_W2 + n * NH + k];
     }
     pk[e] = __float2bfloat16_rn(v);
+  }
+}
+
+// Sums the groups' gradients, clears them for the next batch and adds the
+// batch's loss to *loss; with `step` applies Adam to the FP32 master
+// parameters and rewrites the parameter's bf16 images, otherwise stores the
+// gradient.  32 elements by 8 threads each per CTA.  One pass in place of a
+// cleared gradient, the Adam pass and a repacking pass.
+struct AdamStep {
+  float lr, b1, b2, eps, c1, c2;
+};
+constexpr int RED_W = 32, RED_S = 8;
+__global__ void __launch_bounds__(RED_W* RED_S) reduce_kernel(float* __restrict__ part, int step,
+                                                             AdamStep A, float* __restrict__ prm, float* __restrict__ m,
+                                                             float* __restrict__ v, __nv_bfloat16* __restrict__ pk,
+                                                             float* __restrict__ grad, float* __restrict__ loss) {
+  __shared__ float sum[RED_S][RED_W];
+  const int x = threadIdx.x % RED_W, y = threadIdx.x / RED_W, q = blockIdx.x * RED_W + x;
+  float g = 0.f;
+  if (q < PG_N) {
+#pragma unroll
+    for (int c = y; c < PG_GROUPS; c += RED_S) {
+      g += part[c * PG_N + q];
+      part[c * PG_N + q] = 0.f;
+    }
+  }
+  sum[y][x] = g;
+  __syncthreads();
+  if (y != 0 || q >= PG_N) return;
+  g = 0.f;
+#pragma unroll
+  for (int k = 0; k < RED_S; ++k) g += sum[k][x];
+  if (q == PG_LOSS) {
+    *loss += g;
+    return;
+  }
+  const int i = pg_param(q);
+  if (!step) {
+    grad[i] = g;
+    return;
+  }
+  const float mi = A.b1 * m[i] + (1.f - A.b1) * g;
+  const float vi = A.b2 * v[i] + (1.f - A.b2) * g * g;
+  m[i] = mi;
+  v[i] = vi;
+  const float a = prm[i] - A.lr * (mi * A.c1) / (sqrtf(vi * A.c2) + A.eps);
+  prm[i] = a;
+  const __nv_bfloat16 hi = __float2bfloat16_rn(a), lo = __float2bfloat16_rn(a - bf16_hi(a));
+  if (i < OFF_B1) {
+    const int k = i / NH, n = i % NH;
+    pk[PK_W1B + cm_off(n, k, 16)] = hi;
+    pk[PK_W1B + cm_off(n, k + 5, 16)] = hi;
+    pk[PK_W1B + cm_off(n, k + 9, 16)] = lo;
+  } else if (i >= OFF_W2 && i < OFF_B2) {
+    const int k = (i - OFF_W2) / NH, n = (i - OFF_W2) % NH;
+    pk[PK_W2B + cm_off(n, k, 64)] = hi;
+    pk[PK_W2L + cm_off(n, k, 64)] = lo;
+    pk[PK_W2R + cm_off(k, n, 64)] = hi;
+  } else if (i >= OFF_W3 && i < OFF_B3) {
+    const int n = (i - OFF_W3) / NOUT, k = (i - OFF_W3) % NOUT;
+    pk[PK_W3R + cm_off(n, k, 16)] = hi;
   }
 }
 
@@ -943,10 +1018,12 @@ struct wx_mlp {
   float* prm = nullptr;           // FP32 master parameters [NPARAM]
   float* m = nullptr;             // Adam moments
   float* v = nullptr;
-  float* grad = nullptr;          // FP32 gradient accumulator
+  float* grad = nullptr;          // FP32 gradient
+  float* part = nullptr;          // gradients and losses of the training CTAs' groups [PG_GROUPS][PG_N]
   __nv_bfloat16* pk = nullptr;    // packed bf16 operand images
   float* loss = nullptr;          // device scalar
   int* err = nullptr;             // device error counter (timeouts)
+  int* herr = nullptr;            // pinned copy
   long long step = 0;
   int nsm = 148;
 };
@@ -1022,7 +1099,7 @@ int wx3d_mlp_create(uint64_t seed, wx_mlp** out) {
   cudaDeviceGetAttribute(&w->nsm, cudaDevAttrMultiProcessorCount, dev);
   if (cudaMalloc(&w->prm, NPARAM * 4) || cudaMalloc(&w->m, NPARAM * 4) || cudaMalloc(&w->v, NPARAM * 4) ||
       cudaMalloc(&w->grad, NPARAM * 4) || cudaMalloc(&w->pk, PK_N * 2) || cudaMalloc(&w->loss, 4) ||
-      cudaMalloc(&w->err, 4)) {
+      cudaMalloc(&w->err, 4) || cudaMalloc(&w->part, PG_GROUPS * PG_N * 4) || cudaMallocHost(&w->herr, sizeof(int))) {
     delete w;
     return WX_ERR_CUDA;
   }
@@ -1052,7 +1129,8 @@ int wx3d_mlp_create(uint64_t seed, wx_mlp** out) {
 int wx3d_mlp_destroy(wx_mlp* w) {
   if (!w) return WX_ERR_INVALID_ARG;
   cudaFree(w->prm); cudaFree(w->m); cudaFree(w->v); cudaFree(w->grad); cudaFree(w->pk);
-  cudaFree(w->loss); cudaFree(w->err);
+  cudaFree(w->loss); cudaFree(w->err); cudaFree(w->part);
+  if (w->herr) cudaFreeHost(w->herr);
   delete w;
   return WX_OK;
 }
@@ -1108,8 +1186,11 @@ int wx3d_mlp_forward(wx_mlp* w, int64_t n, const float* d_in, float* d_out, void
   cudaMemsetAsync(w->err, 0, 4, (cudaStream_t)stream);
   forward_kernel<<<grid, TILE, INF_SMEM, (cudaStream_t)stream>>>(d_in, d_out, n, w->pk, w->prm, w->err);
   if (cudaGetLastError() != cudaSuccess) return WX_ERR_CUDA;
-  if (cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess) return WX_ERR_CUDA;
-  return mlp_check(w);
+  // the error count rides on the same synchronisation
+  if (cudaMemcpyAsync(w->herr, w->err, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream) != cudaSuccess ||
+      cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess)
+    return WX_ERR_CUDA;
+  return *w->herr ? WX_ERR_TIMEOUT : WX_OK;
 }
 
 // Mean-squared-error loss and its gradient over all n samples (one pass of
@@ -1119,11 +1200,11 @@ int wx3d_mlp_gradient(wx_mlp* w, int64_t n, const float* d_in, const float* d_tg
   const long long ntiles = (n + TILE - 1) / TILE;
   const int ncta = (int)std::min<long long>(ntiles, w->nsm);
   const int tiles = (int)((ntiles + ncta - 1) / ncta);
-  cudaMemset(w->grad, 0, NPARAM * 4);
   cudaMemset(w->loss, 0, 4);
   cudaMemset(w->err, 0, 4);
-  train_kernel<<<ncta, TILE, train_smem()>>>(d_in, d_tgt, n, 0, tiles, 1.0f / (float)n, w->pk, w->prm, w->grad,
-                                             w->loss, w->err);
+  cudaMemset(w->part, 0, PG_GROUPS * PG_N * 4);
+  train_kernel<<<ncta, TILE, train_smem()>>>(d_in, d_tgt, n, 0, tiles, 1.0f / (float)n, w->pk, w->prm, w->part, w->err);
+  reduce_kernel<<<(PG_N + RED_W - 1) / RED_W, RED_W * RED_S>>>(w->part, 0, AdamStep{}, w->prm, w->m, w->v, w->pk, w->grad, w->loss);
   if (cudaGetLastError() != cudaSuccess) return WX_ERR_CUDA;
   if (cudaDeviceSynchronize() != cudaSuccess) return WX_ERR_CUDA;
   int rc = mlp_check(w);
@@ -1145,20 +1226,20 @@ int wx3d_mlp_train(wx_mlp* w, int64_t n, const float* d_in, const float* d_tgt, 
   const int tiles = (int)((btiles + ncta - 1) / ncta);
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   cudaMemset(w->err, 0, 4);
+  cudaMemset(w->part, 0, PG_GROUPS * PG_N * 4);
   for (int ep = 0; ep < epochs; ++ep) {
     cudaMemset(w->loss, 0, 4);
     long long nb = 0;
     for (long long t0 = 0; t0 < ntiles; t0 += (long long)ncta * tiles, ++nb) {
       const long long cnt = std::min<long long>((long long)ncta * tiles, ntiles - t0) * TILE;
       const long long m = std::min<long long>(cnt, n - t0 * TILE);
-      cudaMemsetAsync(w->grad, 0, NPARAM * 4);
-      train_kernel<<<ncta, TILE, train_smem()>>>(d_in, d_tgt, n, t0, tiles, 1.0f / (float)m, w->pk, w->prm, w->grad,
-                                                 w->loss, w->err);
+      const int parts = (int)std::min<long long>(ncta, (ntiles - t0 + tiles - 1) / tiles);  // CTAs with a tile
+      train_kernel<<<parts, TILE, train_smem()>>>(d_in, d_tgt, n, t0, tiles, 1.0f / (float)m, w->pk, w->prm, w->part,
+                                                  w->err);
       ++w->step;
-      const float c1 = 1.f / (1.f - std::pow(b1, (float)w->step));
-      const float c2 = 1.f / (1.f - std::pow(b2, (float)w->step));
-      adam_kernel<<<(NPARAM + 255) / 256, 256>>>(w->prm, w->grad, w->m, w->v, lr, b1, b2, eps, c1, c2);
-      pack_kernel<<<(PK_N + 255) / 256, 256>>>(w->prm, w->pk);
+      const AdamStep A{lr, b1, b2, eps, 1.f / (1.f - std::pow(b1, (float)w->step)), 1.f / (1.f - std::pow(b2, (float)w->step))};
+      reduce_kernel<<<(PG_N + RED_W - 1) / RED_W, RED_W * RED_S>>>(w->part, 1, A, w->prm, w->m, w->v, w->pk, w->grad,
+                                                                   w->loss);
     }
     if (cudaGetLastError() != cudaSuccess) return WX_ERR_CUDA;
     if (cudaDeviceSynchronize() != cudaSuccess) return WX_ERR_CUDA;
