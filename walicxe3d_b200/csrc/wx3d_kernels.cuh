@@ -1080,12 +1080,27 @@ __global__ void __launch_bounds__(STAGE_THREADS, (corr_ctas_per_sm<NEQ, VISC>())
         state_flux<NEQ, SOLVER, DIR>(l, r, ph, f);
         return Flux<NEQ>(f);
       };
-      {
+      // both ghost layers of plane kk; across an x face to a same-level block
+      // they are two adjacent cells of a row, one 16-byte load per equation
+      // (each of the 32 lanes reads another line there)
+      const bool pair = side < 2 && B.ftype[side] == WX_NEIGH_SAME;
+      const double* row = pair ? gsrc + cell_off(B.fnb[side][0], NEQ, 0, high ? 1 : NC - 1, gj, 1) : nullptr;
+      auto fetch = [&](int kk) {
         double u1[NEQ], u2[NEQ];
-        gather_ghost<NEQ>(gsrc, B, slot, gi, gj, z0, u1);
-        gather_ghost<NEQ>(gsrc, B, slot, oi, oj, z0, u2);
-        take(z0, u1, u2);
-      }
+        if (pair) {
+#pragma unroll
+          for (int e = 0; e < NEQ; ++e) {
+            const double2 v = __ldg(reinterpret_cast<const double2*>(row + (size_t)e * BCELLS + (kk - 1) * PLANE));
+            u1[e] = high ? v.x : v.y;
+            u2[e] = high ? v.y : v.x;
+          }
+        } else {
+          gather_ghost<NEQ>(gsrc, B, slot, gi, gj, kk, u1);
+          gather_ghost<NEQ>(gsrc, B, slot, oi, oj, kk, u2);
+        }
+        take(kk, u1, u2);
+      };
+      fetch(z0);
       plane_barrier();
       for (int m = z0; m <= z1; ++m) {
         const int b = m & 1;
@@ -1098,12 +1113,7 @@ __global__ void __launch_bounds__(STAGE_THREADS, (corr_ctas_per_sm<NEQ, VISC>())
 #pragma unroll
           for (int e = 0; e < NEQ; ++e) S.fy[b][e][(high ? NC * NC : 0) + lane] = f.v[e];
         }
-        if (m < z1) {
-          double u1[NEQ], u2[NEQ];
-          gather_ghost<NEQ>(gsrc, B, slot, gi, gj, m + 1, u1);
-          gather_ghost<NEQ>(gsrc, B, slot, oi, oj, m + 1, u2);
-          take(m + 1, u1, u2);
-        }
+        if (m < z1) fetch(m + 1);
         plane_barrier();
         if (VISC) {
 #pragma unroll
