@@ -511,8 +511,9 @@ def main():
                 # or DMUL takes the issue slot of a DFMA)
                 "inst_frac": (inst * prob.cells / (stage2_ms / 1e3) / (pk * 1e12 / 2)) if (pk and inst) else None,
                 "peak_source": "measured in this run (wx3d_measure_fp64_peak, DFMA chains)",
-                "note": "per-cell figures from the ncu capture on Sedov 256^3; the stage kernels are "
-                        "latency-bound, below both their FP64 instruction bound and the HBM bound"}
+                "note": "per-cell figures from the ncu capture on Sedov 256^3; the stage kernels are bound by "
+                        "instruction issue and the shared-memory data path, below both their FP64 instruction "
+                        "bound and the HBM bound"}
 
     # --- the plain GPU path: the same kernels, one synchronous wx3d_step per
     # step (host round trip each step), default launch shape, no graph ---
@@ -598,7 +599,8 @@ def main():
                                                       "16^3 tile of one persistent launch"}},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": (achieved / peak) if achieved else None, "traffic": traffic,
-                         "kernel": "stage_kernel<ORDER=2> (corrector%s)" % (" + viscous step" if fused else ""),
+                         "kernel": "%s (corrector%s)" % ("stage_kernel<ORDER=2>" if prob.cfg.mhd else "corrector_kernel",
+                                                         " + viscous step" if fused else ""),
                          "peak_source": peak_src, "fp64": fp64,
                          "alg_bytes_per_launch": alg_bytes, "launch_ms": stage2_ms,
                          "step_alg_gbs": step_achieved, "step_frac": step_achieved / peak},
