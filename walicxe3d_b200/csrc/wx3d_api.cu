@@ -301,7 +301,7 @@ struct wx_ctx {
   double* dG = nullptr;
   bool mark_ghosts = false;       // the first-order stage writes dG
   bool g_step = false;            // the step being enqueued writes dG
-  int counters_zeroed = 0;        // stages (bits 1, 2) whose item counter the enqueued work leaves at zero
+  int counters_zeroed = 0;        // stages (bits 1, 2) whose item counter the step begun on the stream left at zero
   bool g_valid = false;           // dG holds the ghosts of the state in dW (with prestep)
   cudaGraphExec_t graph = nullptr;
   bool graph_valid = false;
@@ -606,8 +606,7 @@ int solver_second(wx_ctx* c, bool finish_output) {
   return WX_OK;
 }
 
-// Godunov(order)/LaxFriedrichs + doViscousStep; on return dU holds U^{n+1}.
-int enqueue_solver(wx_ctx* c, bool bump_it, bool finish_output) {
+int enqueue_solver_body(wx_ctx* c, bool bump_it, bool finish_output) {
   const bool src = sources_on(c);
   c->g_step = c->mark_ghosts && c->dG && c->hwind.empty() && c->cfg.solver_type != WX_SOLVER_LAX;
   step_begin_kernel<<<1, 1, 0, c->stream>>>(c->dCtl, c->ph.cfl, c->cfg.cooling_type != WX_COOL_NONE, c->ph.dtout,
@@ -650,6 +649,16 @@ int enqueue_solver(wx_ctx* c, bool bump_it, bool finish_output) {
   }
   if ((rc = solver_first(c))) return rc;
   return solver_second(c, finish_output);
+}
+
+// Godunov(order)/LaxFriedrichs + doViscousStep; on return dU holds U^{n+1}.
+// What the step's first kernel zeroed is good for this step's launches alone:
+// a failure part-way, a single-stage solver or a captured sequence leave
+// nothing for a later one to rely on.
+int enqueue_solver(wx_ctx* c, bool bump_it, bool finish_output) {
+  const int rc = enqueue_solver_body(c, bump_it, finish_output);
+  c->counters_zeroed = 0;
+  return rc;
 }
 
 // mode bits: 1 = hrate, 2 = cooling, 4 = read/write the PRIM buffer, 8 = CFL minimum
@@ -1966,6 +1975,7 @@ int wx3d_step(wx_ctx* c, wx_state* out) {
 int wx3d_run_async(wx_ctx* c, int32_t nsteps) {
   if (!ready(c) || nsteps < 0) return WX_ERR_INVALID_ARG;
   int rc;
+  c->counters_zeroed = 0;   // a replayed graph uses the counters of a wx3d_step_part(0) before it
   if (!c->dt_valid) {
     if ((rc = launch_dt(c, c->dU))) return rc;
     c->dt_valid = true;
