@@ -77,22 +77,31 @@ Kern make_kern() {
   return k;
 }
 
-// Limiters compiled into the corrector: minmod and van Leer (the reference's
-// default) everywhere, the other monotone ones at five equations; NONE,
-// NO_AVERAGE and ALBADA (which fails) use the run-time switch, whose branches
-// sit in every one of the 15 to 24 limiter calls per cell (3,088 blocks of
-// five equations, unfused corrector: UMIST 2.01 -> 0.91 ms, Woodward 2.27 ->
-// 0.82; van Leer at six equations 0.67 -> 0.45, 1,184 blocks).
+// The limiter is compiled into the hydro corrector: a run-time switch puts its
+// branches into every one of the 15 to 24 limiter calls per cell.  Predictor
+// and fused corrector of 1,128 refined blocks, switch -> compiled, at six and
+// at seven equations: UMIST 1.35 -> 0.74 and 2.76 -> 0.96 ms, Woodward 1.50 ->
+// 0.69 and 3.06 -> 0.91, Superbee 1.52 -> 0.70 and 3.08 -> 0.94, NONE 1.04 ->
+// 0.58 and 2.18 -> 0.78; NONE at five 0.79 -> 0.47.
+// MHD keeps the switch for all but minmod and van Leer (the reference's
+// default), where HLLD's arithmetic outweighs it (512 blocks, HLLD: minmod
+// 0.83 ms, UMIST 1.23, Superbee 1.44).
 template <int NEQ, bool MHD, int SOLVER>
 Kern make_kern_lim(int lim) {
-  if constexpr (NEQ == 5) {
-    if (lim == WX_LIMITER_SUPERBEE) return make_kern<NEQ, MHD, SOLVER, WX_LIMITER_SUPERBEE>();
-    if (lim == WX_LIMITER_UMIST) return make_kern<NEQ, MHD, SOLVER, WX_LIMITER_UMIST>();
-    if (lim == WX_LIMITER_WOODWARD) return make_kern<NEQ, MHD, SOLVER, WX_LIMITER_WOODWARD>();
-  }
-  if (lim == WX_LIMITER_VANLEER) return make_kern<NEQ, MHD, SOLVER, WX_LIMITER_VANLEER>();
   if (lim == WX_LIMITER_MINMOD) return make_kern<NEQ, MHD, SOLVER, WX_LIMITER_MINMOD>();
-  return make_kern<NEQ, MHD, SOLVER, LIM_RUNTIME>();
+  if (lim == WX_LIMITER_VANLEER) return make_kern<NEQ, MHD, SOLVER, WX_LIMITER_VANLEER>();
+  if constexpr (MHD) {
+    return make_kern<NEQ, MHD, SOLVER, LIM_RUNTIME>();
+  } else {
+    switch (lim) {
+      case WX_LIMITER_NONE: return make_kern<NEQ, MHD, SOLVER, WX_LIMITER_NONE>();
+      case WX_LIMITER_ALBADA: return make_kern<NEQ, MHD, SOLVER, WX_LIMITER_ALBADA>();
+      case WX_LIMITER_UMIST: return make_kern<NEQ, MHD, SOLVER, WX_LIMITER_UMIST>();
+      case WX_LIMITER_WOODWARD: return make_kern<NEQ, MHD, SOLVER, WX_LIMITER_WOODWARD>();
+      case WX_LIMITER_SUPERBEE: return make_kern<NEQ, MHD, SOLVER, WX_LIMITER_SUPERBEE>();
+      default: return make_kern<NEQ, MHD, SOLVER, WX_LIMITER_NO_AVERAGE>();  // zero slopes, as average()'s default
+    }
+  }
 }
 
 // The source kernel compiled for the radiative runs' source terms
