@@ -69,8 +69,8 @@ struct PhysParams {
   double l_sc, v_sc;
   // derived (derive_phys): 1/mu0; the factors of calcTemp's p/rho (mu0, mui)
   // and of its p/n (EOS_H_RATE); number density per code density for the
-  // table cooling; 1/e_sc
-  double inv_mu0, temp_mu0, temp_mui, temp_n, nd_sc, inv_e_sc;
+  // table cooling
+  double inv_mu0, temp_mu0, temp_mui, temp_n, nd_sc;
   const double* wind;  // nwind x 12: xc yc zc vx vy vz radius mdot vinf temp mu y0 (cgs)
   int32_t nwind;
 };
@@ -123,6 +123,30 @@ __device__ __forceinline__ double mul_rsqrt_nr(double s, double x) {
   return fma(c * e, fma(0.375, e, 0.5), c);
 }
 __device__ __forceinline__ double sqrt_nr(double x) { return mul_rsqrt_nr(x, x); }
+// n / d and sqrt(x) to 0.51 ulp, for results whose last bit a cancellation or
+// an exponential enlarges: the estimate's quotient (root) takes two steps
+// towards a zero residual n - d q (x - s s), five (six) operations after the
+// estimate, in a chain no longer than n rcp_nr(d)'s.  The first step leaves an
+// error of the order of the estimate's squared, the second of its cube.
+// quot_nr takes r ~ 1/d to an ulp and needs one step.
+__device__ __forceinline__ double div_nr(double n, double d) {
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+  const double q0 = n * r;
+  const double q = fma(q0, fma(-d, r, 1.0), q0);
+  return fma(fma(-d, q, n), r, q);
+}
+__device__ __forceinline__ double quot_nr(double n, double d, double r) {
+  const double q = n * r;
+  return fma(fma(-d, q, n), r, q);
+}
+__device__ __forceinline__ double root_nr(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double h = 0.5 * y, s0 = x * y;
+  const double s = fma(fma(-s0, s0, x), h, s0);
+  return fma(fma(-s, s, x), h, s);
+}
 // The same for the discriminant of the fast speeds, which may vanish, or fall
 // below zero by rounding (c_s = c_A along the field): zero there, the
 // library's root for the rest (subnormal, NaN).

@@ -847,8 +847,8 @@ __device__ __forceinline__ void fallback_cell(const SurrParams& P, int id, doubl
     h_cool_step<5>(u, p, dts, ph, &mloss);
   } else {
     const double T = calc_temp<5>(p, ph);
-    const double dh = p[0] * ph.inv_mu0;
-    const double y0 = p[5] * rcp_nr(dh);
+    const double dh = quot_nr(p[0], ph.mu0, ph.inv_mu0);
+    const double y0 = div_nr(p[5], dh);
     const double y1 = h_rate_y1(T, dh, y0, dts);
     p[5] = dh * y1;
     u[5] = p[5];

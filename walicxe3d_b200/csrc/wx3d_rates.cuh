@@ -17,15 +17,18 @@ inline void derive_phys(PhysParams& p) {
   p.temp_mui = p.mui * AMU * p.p_sc / p.d_sc / KB;
   p.temp_n = p.p_sc / KB;
   p.nd_sc = p.d_sc / (p.mui * AMU);
-  p.inv_e_sc = 1.0 / p.e_sc;
 }
 
 // The source terms are chains of divisions, roots, exponentials and
-// logarithms per cell; the divisions are rcp_nr (4 operations against about
-// 12 and a branch), divisions by parameters multiplications by their
-// reciprocals, and the logarithm of T is taken once per temperature:
-// log(c/T) = log c - log T (an absolute error of 1e-15 in a logarithm that
-// is exponentiated or added to O(1) terms).
+// logarithms per cell; a division by a parameter or a temperature is a product
+// by a refined reciprocal (rcp_nr: 4 operations against about 12 and a branch).
+// Where an exponential or the cancellation in the neutral fraction enlarges the
+// last bit, the quotient's or the root's residual is added back (div_nr,
+// quot_nr, root_nr: two operations more), and logarithms are taken of the
+// quotient, not as a difference of logarithms: the errors of a step against
+// 80-bit arithmetic are then those of IEEE divisions and roots, where products
+// alone left a tenth to a third more.  The loss rate itself keeps the products:
+// it enters a step weakly (5 to 10 % more error in the rate, 1 % in the step).
 
 // calcTemp (hydro_core.f90:231-270); EOS >= 0 fixes the equation of state
 // at compile time, -1 reads it from ph.
@@ -34,13 +37,13 @@ __device__ __forceinline__ double calc_temp(const double* p, const PhysParams& p
   double temp = 0.0;
   switch (EOS >= 0 ? EOS : ph.eos) {
     case WX_EOS_ADIABATIC:
-    case WX_EOS_SINGLE_SPECIE: temp = p[4] * rcp_nr(p[0]) * ph.temp_mu0; break;
+    case WX_EOS_SINGLE_SPECIE: temp = div_nr(p[4], p[0]) * ph.temp_mu0; break;
     case WX_EOS_TWOTEMP:
-      temp = p[4] * rcp_nr(p[0]);
+      temp = div_nr(p[4], p[0]);
       temp = temp * ph.temp_mu0 > ph.ion_thres ? temp * ph.temp_mui : temp * ph.temp_mu0;
       break;
     case WX_EOS_H_RATE:
-      if (ph.npassive >= 1) temp = p[4] * rcp_nr(2.0 * p[0] * ph.inv_mu0 - p[FP]) * ph.temp_n;
+      if (ph.npassive >= 1) temp = div_nr(p[4], 2.0 * quot_nr(p[0], ph.mu0, ph.inv_mu0) - p[FP]) * ph.temp_n;
       break;
   }
   return temp;
@@ -50,18 +53,18 @@ __device__ __forceinline__ double calc_temp(const double* p, const PhysParams& p
 // fraction y1 for the cell's temperature T and H density dh.
 __device__ __forceinline__ double h_rate_y1(double T, double dh, double y0, double dts) {
   const double xi = 1.e-4;
-  const double LN_1E4 = 9.210340371976184;
-  const double col = 5.83e-11 * sqrt_nr(T) * exp(-157828. * rcp_nr(T));   // colf, hrate.f90:73
-  const double rec = 2.55e-13 * exp(0.79 * (LN_1E4 - log(T)));           // alpha, hrate.f90:58: (1e4/T)^0.79
+  const double Tm = rcp_nr(T);
+  const double col = 5.83e-11 * sqrt_nr(T) * exp(quot_nr(-157828., T, Tm));   // colf, hrate.f90:73
+  const double rec = 2.55e-13 * exp(0.79 * log(1.e4 * Tm));        // alpha, hrate.f90:58: (1e4/T)^0.79
   const double a = rec + col;
   const double b = -((2.0 + xi) * rec + (1.0 + xi) * col + 0.0);
   const double c = (1.0 + xi) * rec;
-  const double d = sqrt_nr(b * b - 4.0 * a * c);
+  const double d = root_nr(b * b - 4.0 * a * c);
   // g0 = gn / gd; (1 + g0 e) / (1 - g0 e) = (gd + gn e) / (gd - gn e)
   const double gn = 2.0 * a * y0 + b + d, gd = 2.0 * a * y0 + b - d;
   const double e = exp(-d * dh * dts);
-  const double q = (gd + gn * e) * rcp_nr(gd - gn * e);
-  double y1 = (-b - d * q) * rcp_nr(2.0 * a);
+  const double q = div_nr(gd + gn * e, gd - gn * e);
+  double y1 = div_nr(-b - d * q, 2.0 * a);
   y1 = dmin(y1, 1.0 - xi);
   y1 = dmax(y1, 0.0);
   return y1;
@@ -75,7 +78,9 @@ __device__ __forceinline__ double aloss_h(double x1, double den, double dH0, dou
   const double C0 = 0.5732, C1 = 1.8288e-5, C2 = -1.15822e-10, C3 = 9.4288e-16;
   const double D0 = 0.5856, D1 = 1.55083e-5, D2 = -9.669e-12, D3 = 5.716e-19;
   const double ENK = 118409., EN = 1.634E-11;
-  const double LN_157890 = 11.969653867015934, LN_1E5 = 11.512925464970229;
+  const double BETAH = 2.85136357582834029e-27;  // 1.133e-24 / sqrt(157890)
+  const double LN_A = 0.456728402045705915;         // ln 1.5789
+  const double EQUIL = 7.40157317573616216e-22;  // 1.0455e-18 / 1e5^0.63
   const double Te = dmax(Te0, 10.);
   const double dHp = (1. - x1) * den;
   const double de = dHp + 1.E-4 * den;
@@ -89,7 +94,7 @@ __device__ __forceinline__ double aloss_h(double x1, double den, double dH0, dou
     const double frac = (Te - 55000.) / 17000.;
     omega = (1. - frac) * oL + frac * oH;
   }
-  const double Tm = rcp_nr(Te), lT = log(Te);
+  const double Tm = rcp_nr(Te), lx = log(Te * 1.E-5);  // one logarithm for the warp's cold and hot cells
   const double sTe = sqrt_nr(Te);
   const double qla = 8.6287E-6 * 0.5 * (sTe * Tm) * omega * exp(-ENK * Tm);
   const double ecoll = dmax(de * dH0 * qla * EN, 0.);
@@ -103,18 +108,19 @@ __device__ __forceinline__ double aloss_h(double x1, double den, double dH0, dou
     fr = 0.5 * (1. + (1. - ex2) * rcp_nr(1. + ex2));
   }
   if (fr < 1.) {  // recombination and the O I, O II lines
-    // betah: a = 157890/T; a^-1/2 and a^-0.33333 = exp(-0.33333 ln a)
-    const double la = LN_157890 - lT;
-    const double betah = 1.133e-24 * sqrt_nr(Te * (1. / 157890.)) * (-0.0713 + 0.5 * la + 0.640 * exp(-0.33333 * la));
+    // betah: a = 157890/T; 1.133e-24 a^-1/2 = 2.85...e-27 T^1/2 and
+    // a^-0.33333 = exp(-0.33333 ln a)
+    const double la = LN_A - lx;
+    const double betah = BETAH * sTe * (-0.0713 + 0.5 * la + 0.640 * exp(-0.33333 * la));
     const double erec = dmax(de * dHp * betah, 0.);
     const double Tm2 = Tm * Tm;
     const double eOI = dmax(de * (XO * dH0) * exp10(1381465 * Tm2 - 12328.69 * Tm - 19.82621), 0.);
     const double eOII = dmax(de * (XO * dHp) * exp10(-2061075. * Tm2 - 14596.24 * Tm - 19.01402), 0.);
     loss += (erec + 7.033 * (eOI + eOII)) * (1. - fr);
   }
-  if (fr > 0.) {  // equilibrium losses; Te^-0.63 and (Te 1e-5)^1.63 as exp(a ln x)
+  if (fr > 0.) {  // equilibrium losses; with x = Te 1e-5, x^1.63 and Te^-0.63 = 1e5^-0.63 x^-0.63 as exp(a ln x)
     const double HIIcool = de * dHp * (1.3 * 1.42E-27 * sTe);
-    const double equil = 1.0455E-18 * exp(-0.63 * lT) * (1. - exp(-exp(1.63 * (lT - LN_1E5)))) * de * den + HIIcool;
+    const double equil = EQUIL * exp(-0.63 * lx) * (1. - exp(-exp(1.63 * lx))) * de * den + HIIcool;
     loss += equil * fr;
   }
   return loss;
@@ -200,16 +206,16 @@ __device__ __forceinline__ double get_lambda_schure(const double* __restrict__ T
 // and u the old neutral density.
 template <int FP, int EOS = -1>
 __device__ __forceinline__ void cool_h_cell(double* u, double* p, double dts, const PhysParams& ph, double& mloss) {
-  const double dh = p[0] * ph.inv_mu0;
+  const double dh = quot_nr(p[0], ph.mu0, ph.inv_mu0);
   const double dh0 = p[FP];
-  const double y0 = ph.mu0 * u[FP] * rcp_nr(u[0]);
+  const double y0 = div_nr(ph.mu0 * u[FP], u[0]);
   u[FP] = p[FP];
   const double Temp = calc_temp<FP, EOS>(p, ph);
   if (Temp > 1.e4) {
     const double L0 = aloss_h(y0, dh, dh0, Temp);
-    const double ce = (2.0 * L0) * rcp_nr(3.0 * KB * dh * Temp);
+    const double ce = div_nr(2.0 * L0, 3.0 * KB * dh * Temp);
     const double T1 = 10.0 + (Temp - 10.0) * exp(-ce * dts);
-    double cf = T1 * rcp_nr(Temp);
+    double cf = div_nr(T1, Temp);
     mloss = dmax(mloss, 1.0 - cf);
     if (cf < 1.0 - ph.cooling_limit) cf = 1.0 - ph.cooling_limit;
     if (Temp * cf < 10.0) cf = 10.0 / Temp;
@@ -226,8 +232,8 @@ __device__ __forceinline__ void cool_h_cell(double* u, double* p, double dts, co
 template <int FP>
 __device__ __forceinline__ void h_cool_step(double* u, double* p, double dts, const PhysParams& ph, double* mloss) {
   const double T = calc_temp<FP, WX_EOS_H_RATE>(p, ph);
-  const double dh = p[0] * ph.inv_mu0;
-  const double y0 = p[FP] * rcp_nr(dh);
+  const double dh = quot_nr(p[0], ph.mu0, ph.inv_mu0);
+  const double y0 = div_nr(p[FP], dh);
   p[FP] = dh * h_rate_y1(T, dh, y0, dts);
   cool_h_cell<FP, WX_EOS_H_RATE>(u, p, dts, ph, *mloss);
 }
@@ -264,7 +270,7 @@ __device__ __forceinline__ void table_cooling(double* u, double* p, double dts, 
         al = find_coef(cool_lt, cool_lc, ncool, logT);
       }
       const double nd = p[0] * ph.nd_sc;
-      const double ce = al * (nd * nd) * (rcp_nr(ETH) * ph.inv_e_sc);
+      const double ce = div_nr(al * (nd * nd), ETH * ph.e_sc);
       double cf = exp(-ce * dts);
       mloss = dmax(mloss, 1.0 - cf);
       if (cf < 1.0 - ph.cooling_limit) cf = 1.0 - ph.cooling_limit;

@@ -34,12 +34,13 @@ struct SrcParams {
 // fixes the source terms at compile time for the two combinations of the
 // radiative runs (1: EOS_H_RATE + COOL_H, 2: EOS_H_RATE + COOL_TABLE), which
 // leaves the other branches out of the register allocation; 0 reads the
-// equation of state and the cooling type from ph.  With Newton-type
-// reciprocals for its some twenty divisions a cell, one logarithm per
-// temperature, a guessed table row and the loss terms of zero weight left
-// out: 20,896-block winds mesh 3.51 -> 2.30 ms, 4,712-block remnant of hot
-// gas 1.30 -> 0.77 ms (three, four and six CTAs per SM: 0.76, 0.76 and 0.79
-// ms there, 20, 7 and 6 % slower on the winds).
+// equation of state and the cooling type from ph.  With refined reciprocals
+// for its some twenty divisions a cell, one logarithm per temperature in the
+// loss rate, a guessed table row and the loss terms of zero weight left out:
+// 20,896-block winds mesh 3.51 -> 2.39 ms, 4,712-block remnant of hot gas 1.30
+// -> 0.78 ms.  Five CTAs per SM leave 48 registers: COOL_H spills 536 bytes,
+// COOL_TABLE 56, and three, four and six CTAs measured 0.76, 0.76 and 0.79 ms
+// on the remnant, 20, 7 and 6 % more than five on the winds.
 template <int NEQ, bool MHD, int SPEC = 0>
 __global__ void __launch_bounds__(256, 5) source_kernel(SrcParams P) {
   constexpr int FP = MHD ? 8 : 5;
@@ -80,8 +81,8 @@ __global__ void __launch_bounds__(256, 5) source_kernel(SrcParams P) {
         h_cool_step<FP>(u, p, dts, ph, &mloss);  // hrate.f90:101-140 then cooling_h.f90:175-246
       } else if (HAS_PAS && do_hrate && eos == WX_EOS_H_RATE) {  // hrate.f90:101-140
         const double T = calc_temp<FP, EOS_C>(p, ph);
-        const double dh = p[0] * ph.inv_mu0;
-        const double y0 = p[fp] * rcp_nr(dh);
+        const double dh = quot_nr(p[0], ph.mu0, ph.inv_mu0);
+        const double y0 = div_nr(p[fp], dh);
         const double y1 = h_rate_y1(T, dh, y0, dts);
         p[fp] = dh * y1;
         if (cooling != WX_COOL_H) u[fp] = p[fp];
