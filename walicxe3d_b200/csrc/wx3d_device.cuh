@@ -295,30 +295,43 @@ __device__ __forceinline__ double average_t(double a, double b, int opt) {
 // ---------------------------------------------------------------------------
 // Riemann solvers along x of permuted primitive states.
 
-// HLL with the sound speeds supplied by the caller (hll.f90:175-260), as
-//   F = (sr G_L - sl G_R) / (sr - sl),  G_K = F_K - s_K U_K
+// HLL with the sound speeds supplied by the caller (hll.f90:175-260):
+//   F = wl F_L + wr F_R + w (U_R - U_L),  wl = sr / (sr - sl), wr = 1 - wl,
+//   w = sl wl
 // with sl and sr clamped to sl <= 0 <= sr: a supersonic interface then gives
-// G_K = F_K of the upwind side with weight one, so there is no branch, and
-// G takes fewer operations than F and U.
+// the upwind side's flux with weight exactly one, so there is no branch.  In
+// slow flow the two sides nearly cancel, so U_R - U_L is taken of the states
+// themselves for the mass m, the thermal energy and the passive scalars; the
+// momenta and the kinetic energy, whose coefficients g_K = rho_K (w_K u_K -+ w)
+// add up to m, are the upwind value (side A of m's sign) carried by m and a
+// correction, g_L q_L + g_R q_R = m q_A + g_B (q_B - q_A).
+// As sums g_L q_L + g_R q_R throughout, the mass flux was off by an ulp of
+// rho c instead of rho u (130 times the error at Mach 0.01, 4 times at 0.3)
+// and the momenta by 2 to 3 times; the error against 80-bit arithmetic is now
+// that of F_K and U_K spelt out in 64 bits, or less.
 template <int NEQ>
 __device__ __forceinline__ void riemann_hll_c(const double* pL, const double* pR, double cl, double cr, double* f,
                                               double cv) {
   const double sl = dmin(dmin(pL[1] - cl, pR[1] - cr), 0.0);
   const double sr = dmax(dmax(pL[1] + cl, pR[1] + cr), 0.0);
-  const double inv = rcp_nr(sr - sl);
-  const double wl = sr * inv, wr = -sl * inv;
-  // side by side: s is the wave speed of G_L (sl) and of G_R (sr)
-  const double al = pL[1] - sl, ar = pR[1] - sr;
-  const double gl = pL[0] * al * wl, gr = pR[0] * ar * wr;
+  const double wl = div_nr(sr, sr - sl), wr = 1.0 - wl, w = sl * wl;
+  const double xl = wl * pL[1], xr = wr * pR[1];
+  const double m = xl * pL[0] + xr * pR[0] + w * (pR[0] - pL[0]);
+  const bool left = m >= 0.0;
+  const double g = (left ? pR[0] : pL[0]) * ((left ? xr : xl) + (left ? w : -w));
   const double kl = pL[1] * pL[1] + pL[2] * pL[2] + pL[3] * pL[3];
   const double kr = pR[1] * pR[1] + pR[2] * pR[2] + pR[3] * pR[3];
-  f[0] = gl + gr;
-  f[1] = gl * pL[1] + gr * pR[1] + (wl * pL[4] + wr * pR[4]);
-  f[2] = gl * pL[2] + gr * pR[2];
-  f[3] = gl * pL[3] + gr * pR[3];
-  f[4] = 0.5 * (gl * kl + gr * kr) + (wl * pL[4] * (cv * al + pL[1]) + wr * pR[4] * (cv * ar + pR[1]));
+  auto carried = [&](double l, double r) {
+    const double a = left ? l : r, b = left ? r : l;
+    return m * a + g * (b - a);
+  };
+  f[0] = m;
+  f[1] = carried(pL[1], pR[1]) + (wl * pL[4] + wr * pR[4]);
+  f[2] = carried(pL[2], pR[2]);
+  f[3] = carried(pL[3], pR[3]);
+  f[4] = 0.5 * carried(kl, kr) + ((cv + 1.0) * (xl * pL[4] + xr * pR[4]) + cv * (w * (pR[4] - pL[4])));
 #pragma unroll
-  for (int e = 5; e < NEQ; ++e) f[e] = wl * al * pL[e] + wr * ar * pR[e];
+  for (int e = 5; e < NEQ; ++e) f[e] = xl * pL[e] + xr * pR[e] + w * (pR[e] - pL[e]);
 }
 
 // HLLC with the sound speeds supplied by the caller (hllc.f90:209-357).  The
