@@ -150,7 +150,7 @@ __device__ __forceinline__ double root_nr(double x) {
 // The same for the discriminant of the fast speeds, which may vanish, or fall
 // below zero by rounding (c_s = c_A along the field): zero there, the
 // library's root for the rest (subnormal, NaN).
-__device__ __forceinline__ double sqrt_nn(double x) { return x > 1.0e-290 ? sqrt_nr(x) : (x <= 0.0 ? 0.0 : sqrt(x)); }
+__device__ __forceinline__ double sqrt_nn(double x) { return x > 1.0e-290 ? root_nr(x) : (x <= 0.0 ? 0.0 : sqrt(x)); }
 // Sound speed sqrt(gp / rho), gp = gamma p, as gp / sqrt(gp rho): one
 // estimate and no reciprocal of rho.
 __device__ __forceinline__ double sound_nr(double gp, double rho) { return mul_rsqrt_nr(gp, gp * rho); }
@@ -231,8 +231,8 @@ __device__ __forceinline__ void xflux(const double* p, double* f, double cv) {
 __device__ __forceinline__ double cfastX(const double* p, double g) {
   const double b2 = p[5] * p[5] + p[6] * p[6] + p[7] * p[7];
   const double rinv = rcp_nr(p[0]);
-  const double a = (g * p[4] + b2) * rinv;
-  return sqrt_nr(0.5 * (a + sqrt_nn(a * a - 4. * g * p[4] * (p[5] * p[5]) * rinv * rinv)));
+  const double a = quot_nr(g * p[4] + b2, p[0], rinv);
+  return root_nr(0.5 * (a + sqrt_nn(a * a - 4. * g * p[4] * (p[5] * p[5]) * rinv * rinv)));
 }
 
 // average (hydro_core.f90:640-699)
@@ -442,8 +442,11 @@ __device__ __forceinline__ void riemann_hlld(const double* pl, const double* pr,
   const double slmul = sl - pl[1];
   const double srmur = sr - pr[1];
   const double den = srmur * pr[0] - slmul * pl[0];
+  // the fast speeds, the contact's speed and the pressure between the fast
+  // waves enter every flux: with their residuals added back the x-momentum flux
+  // rounds as with IEEE divisions and roots (1.07 times its error without)
   const double rden = rcp_nr(den);
-  const double sM = (srmur * (pr[0] * pr[1]) - slmul * (pl[0] * pl[1]) - pTR + pTL) * rden;
+  const double sM = quot_nr(srmur * (pr[0] * pr[1]) - slmul * (pl[0] * pl[1]) - pTR + pTL, den, rden);
   const double srmsM = sr - sM;
   const double slmsM = sl - sM;
   const double rsl = rcp_nr(slmsM), rsr = rcp_nr(srmsM);
@@ -452,7 +455,7 @@ __device__ __forceinline__ void riemann_hlld(const double* pl, const double* pr,
   const double sqrl = sqrt_nr(rhostl), sqrr = sqrt_nr(rhostr);
   const double sstl = sM - mul_rsqrt_nr(fabs(bx), rhostl);
   const double sstr = sM + mul_rsqrt_nr(fabs(bx), rhostr);
-  const double pst = (srmur * pr[0] * pTL - slmul * pl[0] * pTR + pl[0] * pr[0] * srmur * slmul * (pr[1] - pl[1])) * rden;
+  const double pst = quot_nr(srmur * pr[0] * pTL - slmul * pl[0] * pTR + pl[0] * pr[0] * srmur * slmul * (pr[1] - pl[1]), den, rden);
   const bool leftside = (sstl >= 0.0) || (!(sstr <= 0.0) && (sM >= 0.0));
   // star state of the left or right side
   double vstl = 0, wstl = 0, bystl = 0, bzstl = 0, vstr = 0, wstr = 0, bystr = 0, bzstr = 0;
