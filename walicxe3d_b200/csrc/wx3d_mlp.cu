@@ -348,6 +348,7 @@ __device__ void load_weights(S& s, const __nv_bfloat16* __restrict__ pk, const f
 constexpr int PG_GROUPS = 16;
 constexpr int PG_W3 = NH * (NH + 1), PG_W1 = PG_W3 + NOUT * (NH + 1), PG_LOSS = PG_W1 + (NIN + 1) * NH, PG_N = PG_LOSS + 1;
 static_assert(PG_LOSS == NPARAM, "one gradient element per parameter");
+constexpr size_t PART_BYTES = (PG_GROUPS * PG_N + 2) * 4;  // and the loss and the error count, cleared with them
 
 // The parameter of gradient element q.
 __device__ __forceinline__ int pg_param(int q) {
@@ -1019,11 +1020,10 @@ struct wx_mlp {
   float* m = nullptr;             // Adam moments
   float* v = nullptr;
   float* grad = nullptr;          // FP32 gradient
-  float* part = nullptr;          // gradients and losses of the training CTAs' groups [PG_GROUPS][PG_N]
+  float* part = nullptr;          // gradients and losses of the training CTAs' groups [PG_GROUPS][PG_N]; then loss, err
   __nv_bfloat16* pk = nullptr;    // packed bf16 operand images
   float* loss = nullptr;          // device scalar
   int* err = nullptr;             // device error counter (timeouts)
-  int* herr = nullptr;            // pinned copy
   long long step = 0;
   int nsm = 148;
 };
@@ -1098,8 +1098,7 @@ int wx3d_mlp_create(uint64_t seed, wx_mlp** out) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&w->nsm, cudaDevAttrMultiProcessorCount, dev);
   if (cudaMalloc(&w->prm, NPARAM * 4) || cudaMalloc(&w->m, NPARAM * 4) || cudaMalloc(&w->v, NPARAM * 4) ||
-      cudaMalloc(&w->grad, NPARAM * 4) || cudaMalloc(&w->pk, PK_N * 2) || cudaMalloc(&w->loss, 4) ||
-      cudaMalloc(&w->err, 4) || cudaMalloc(&w->part, PG_GROUPS * PG_N * 4) || cudaMallocHost(&w->herr, sizeof(int))) {
+      cudaMalloc(&w->grad, NPARAM * 4) || cudaMalloc(&w->pk, PK_N * 2) || cudaMalloc(&w->part, PART_BYTES)) {
     delete w;
     return WX_ERR_CUDA;
   }
@@ -1117,6 +1116,8 @@ int wx3d_mlp_create(uint64_t seed, wx_mlp** out) {
   cudaMemcpy(w->prm, h.data(), NPARAM * 4, cudaMemcpyHostToDevice);
   cudaMemset(w->m, 0, NPARAM * 4);
   cudaMemset(w->v, 0, NPARAM * 4);
+  w->loss = w->part + PG_GROUPS * PG_N;
+  w->err = reinterpret_cast<int*>(w->loss + 1);
   cudaMemset(w->err, 0, 4);
   pack_kernel<<<(PK_N + 255) / 256, 256>>>(w->prm, w->pk);
   if (cudaDeviceSynchronize() != cudaSuccess) { delete w; return WX_ERR_CUDA; }
@@ -1129,8 +1130,7 @@ int wx3d_mlp_create(uint64_t seed, wx_mlp** out) {
 int wx3d_mlp_destroy(wx_mlp* w) {
   if (!w) return WX_ERR_INVALID_ARG;
   cudaFree(w->prm); cudaFree(w->m); cudaFree(w->v); cudaFree(w->grad); cudaFree(w->pk);
-  cudaFree(w->loss); cudaFree(w->err); cudaFree(w->part);
-  if (w->herr) cudaFreeHost(w->herr);
+  cudaFree(w->part);
   delete w;
   return WX_OK;
 }
@@ -1186,11 +1186,13 @@ int wx3d_mlp_forward(wx_mlp* w, int64_t n, const float* d_in, float* d_out, void
   cudaMemsetAsync(w->err, 0, 4, (cudaStream_t)stream);
   forward_kernel<<<grid, TILE, INF_SMEM, (cudaStream_t)stream>>>(d_in, d_out, n, w->pk, w->prm, w->err);
   if (cudaGetLastError() != cudaSuccess) return WX_ERR_CUDA;
-  // the error count rides on the same synchronisation
-  if (cudaMemcpyAsync(w->herr, w->err, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream) != cudaSuccess ||
+  // the copy of the error count is the call's one wait (a pinned word for it
+  // took 2.3 ms to allocate, more than twenty calls)
+  int e = 0;
+  if (cudaMemcpyAsync(&e, w->err, sizeof(int), cudaMemcpyDeviceToHost, (cudaStream_t)stream) != cudaSuccess ||
       cudaStreamSynchronize((cudaStream_t)stream) != cudaSuccess)
     return WX_ERR_CUDA;
-  return *w->herr ? WX_ERR_TIMEOUT : WX_OK;
+  return e ? WX_ERR_TIMEOUT : WX_OK;
 }
 
 // Mean-squared-error loss and its gradient over all n samples (one pass of
@@ -1200,9 +1202,7 @@ int wx3d_mlp_gradient(wx_mlp* w, int64_t n, const float* d_in, const float* d_tg
   const long long ntiles = (n + TILE - 1) / TILE;
   const int ncta = (int)std::min<long long>(ntiles, w->nsm);
   const int tiles = (int)((ntiles + ncta - 1) / ncta);
-  cudaMemset(w->loss, 0, 4);
-  cudaMemset(w->err, 0, 4);
-  cudaMemset(w->part, 0, PG_GROUPS * PG_N * 4);
+  cudaMemset(w->part, 0, PART_BYTES);
   train_kernel<<<ncta, TILE, train_smem()>>>(d_in, d_tgt, n, 0, tiles, 1.0f / (float)n, w->pk, w->prm, w->part, w->err);
   reduce_kernel<<<(PG_N + RED_W - 1) / RED_W, RED_W * RED_S>>>(w->part, 0, AdamStep{}, w->prm, w->m, w->v, w->pk, w->grad, w->loss);
   if (cudaGetLastError() != cudaSuccess) return WX_ERR_CUDA;
@@ -1225,10 +1225,9 @@ int wx3d_mlp_train(wx_mlp* w, int64_t n, const float* d_in, const float* d_tgt, 
   const int ncta = (int)std::min<long long>(btiles, w->nsm);
   const int tiles = (int)((btiles + ncta - 1) / ncta);
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-  cudaMemset(w->err, 0, 4);
-  cudaMemset(w->part, 0, PG_GROUPS * PG_N * 4);
+  cudaMemset(w->part, 0, PART_BYTES);
   for (int ep = 0; ep < epochs; ++ep) {
-    cudaMemset(w->loss, 0, 4);
+    if (ep) cudaMemset(w->loss, 0, 4);
     long long nb = 0;
     for (long long t0 = 0; t0 < ntiles; t0 += (long long)ncta * tiles, ++nb) {
       const long long cnt = std::min<long long>((long long)ncta * tiles, ntiles - t0) * TILE;
