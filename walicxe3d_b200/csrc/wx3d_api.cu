@@ -1464,8 +1464,10 @@ static int copy_blocks(wx_ctx* c, int32_t array, int32_t n, const int32_t* slots
   const size_t block = (size_t)c->neq * BCELLS;
   // the kernel takes 16-byte aligned buffers that lie in one allocation of
   // this context's device, and each slot once when it writes them; other
-  // calls copy block by block, in order, with the copies' own checks
-  bool one_launch = n > 0 && reinterpret_cast<uintptr_t>(buf) % 16 == 0 && device_range(c->dev, buf, block * 8 * (size_t)n);
+  // calls copy block by block, in order, with the copies' own checks, and so
+  // does a single block (22 us; 25 with the look at the buffer and a launch,
+  // from two blocks on the kernel wins: 24 against 27)
+  bool one_launch = n > 1 && reinterpret_cast<uintptr_t>(buf) % 16 == 0 && device_range(c->dev, buf, block * 8 * (size_t)n);
   if (one_launch && !pack) {
     std::vector<char> seen(c->max_blocks, 0);
     for (int b = 0; b < n; ++b) {
