@@ -1801,18 +1801,26 @@ int wx3d_read_state(wx_ctx* c, const char* path, int32_t* noutput, char* datadir
   return WX_OK;
 }
 
-// The physical cells U(1:ns, :, 1:16, 1:16, kf) of a plane of the Fortran
-// array, to or from the staging slab [j][i][eq][nbmax], and nothing else: the
-// ghosts and the entries past ns neither travel nor change.  Where every
-// entry travels, a row of 16 cells is one contiguous run.
-static cudaError_t copy_fortran_plane(wx_ctx* c, int nbmax, int ns, int kf, double* U, bool up) {
+// How a plane's physical cells U(:, :, 1:16, 1:16, kf) of the Fortran array
+// travel to or from the staging slab [j][i][eq][nbmax].  The ghosts never do,
+// and a download changes neither them nor the entries past ns.
+enum class PlaneCopy {
+  ROWS,     // rows of 16 cells with all nbmax entries: long contiguous runs
+  SPAN,     // the contiguous run from the first to the last physical cell, up only (slab rows of 20 cells)
+  STRIDED,  // entries 1..ns of every cell
+};
+
+static cudaError_t copy_fortran_plane(wx_ctx* c, int nbmax, int ns, int kf, double* U, bool up, PlaneCopy how,
+                                      int row = NC) {
   double* h = U + (size_t)nbmax * c->neq * (400 * (size_t)(kf + 1) + 20 * 2 + 2);
   const size_t cell = (size_t)nbmax * c->neq * 8;   // bytes of one cell's entries
+  if (how == PlaneCopy::SPAN)
+    return cudaMemcpyAsync(c->dStage, h, cell * (15 * 20 + 16), cudaMemcpyHostToDevice, c->stream);
   cudaMemcpy3DParms p{};
-  const bool rows = ns == nbmax;
+  const bool rows = how == PlaneCopy::ROWS;
   const cudaPitchedPtr host = rows ? make_cudaPitchedPtr(h, 20 * cell, 20 * cell, 20)
                                    : make_cudaPitchedPtr(h, (size_t)nbmax * 8, (size_t)nbmax * 8, 20 * (size_t)c->neq);
-  const cudaPitchedPtr dev = rows ? make_cudaPitchedPtr(c->dStage, 16 * cell, 16 * cell, 16)
+  const cudaPitchedPtr dev = rows ? make_cudaPitchedPtr(c->dStage, row * cell, row * cell, 16)
                                   : make_cudaPitchedPtr(c->dStage, (size_t)nbmax * 8, (size_t)nbmax * 8, 16 * (size_t)c->neq);
   p.srcPtr = up ? host : dev;
   p.dstPtr = up ? dev : host;
@@ -1821,14 +1829,40 @@ static cudaError_t copy_fortran_plane(wx_ctx* c, int nbmax, int ns, int kf, doub
   return cudaMemcpy3DAsync(&p, c->stream);
 }
 
+static bool pageable(const void* p) {
+  cudaPointerAttributes at{};
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return at.type == cudaMemoryTypeUnregistered;
+}
+
+// One call per plane carries up to 64 KB of pageable memory up without a wait
+// (4 entries of five equations: 165 us; 198 as 16 rows).
+static bool small_span(const double* U, int nbmax, int neq) {
+  return (size_t)nbmax * neq * (15 * 20 + 16) * 8 <= 65536 && pageable(U);
+}
+
+// Short strided rows are fast only where rows and pitch are whole 64-byte
+// lines (8 of 16 entries, an upload: 246 us against 358 with whole planes; 3
+// of 4: 3005 against 167 pageable and 670 against 205 pinned).
+static bool line_strides(const double* U, int nbmax, int ns) {
+  return ns < nbmax && ns % 8 == 0 && nbmax % 8 == 0 && reinterpret_cast<uintptr_t>(U) % 64 == 0;
+}
+
 int wx3d_upload_U_fortran(wx_ctx* c, int32_t nbmax, const double* U) {
   if (!c || !U || nbmax <= 0) return WX_ERR_INVALID_ARG;
   const int ns = std::min(nbmax, c->max_blocks);
+  const PlaneCopy how = small_span(U, nbmax, c->neq) ? PlaneCopy::SPAN
+                        : line_strides(U, nbmax, ns) ? PlaneCopy::STRIDED
+                                                     : PlaneCopy::ROWS;
+  const int row = how == PlaneCopy::SPAN ? 20 : NC;
   int rc;
-  if ((rc = ensure_stage(c, (size_t)nbmax * c->neq * PLANE * 8))) return rc;
+  if ((rc = ensure_stage(c, (size_t)nbmax * c->neq * row * NC * 8))) return rc;
   for (int kf = 1; kf <= NC; ++kf) {
-    WX_CUDA(copy_fortran_plane(c, nbmax, ns, kf, const_cast<double*>(U), true));
-    fortran_to_native<<<c->nsm * 4, 256, 0, c->stream>>>(c->dStage, c->dU, nbmax, ns, c->neq, kf);
+    WX_CUDA(copy_fortran_plane(c, nbmax, ns, kf, const_cast<double*>(U), true, how));
+    fortran_to_native<<<c->nsm * 4, 256, 0, c->stream>>>(c->dStage, c->dU, nbmax, ns, c->neq, kf, row);
     WX_LAUNCHED();
   }
   WX_CUDA(cudaStreamSynchronize(c->stream));
@@ -1841,12 +1875,22 @@ int wx3d_upload_U_fortran(wx_ctx* c, int32_t nbmax, const double* U) {
 int wx3d_download_U_fortran(wx_ctx* c, int32_t nbmax, double* U) {
   if (!c || !U || nbmax <= 0) return WX_ERR_INVALID_ARG;
   const int ns = std::min(nbmax, c->max_blocks);
+  // fewer slots than entries: pinned memory takes the strided rows at any
+  // size, pageable memory where they are whole lines; elsewhere the rows come
+  // up first, so that they can go back whole (3 of 4 entries: 7664 us strided,
+  // 573 with whole planes up and down)
+  const bool strided = ns < nbmax && (line_strides(U, nbmax, ns) || !pageable(U));
+  const PlaneCopy how = strided ? PlaneCopy::STRIDED : PlaneCopy::ROWS;
+  const bool first_up = ns < nbmax && !strided;
+  const PlaneCopy up = first_up && small_span(U, nbmax, c->neq) ? PlaneCopy::SPAN : how;
+  const int row = up == PlaneCopy::SPAN ? 20 : NC;
   int rc;
-  if ((rc = ensure_stage(c, (size_t)nbmax * c->neq * PLANE * 8))) return rc;
+  if ((rc = ensure_stage(c, (size_t)nbmax * c->neq * row * NC * 8))) return rc;
   for (int kf = 1; kf <= NC; ++kf) {
-    native_to_fortran<<<c->nsm * 4, 256, 0, c->stream>>>(c->dU, c->dStage, nbmax, ns, c->neq, kf);
+    if (first_up) WX_CUDA(copy_fortran_plane(c, nbmax, ns, kf, U, true, up));
+    native_to_fortran<<<c->nsm * 4, 256, 0, c->stream>>>(c->dU, c->dStage, nbmax, ns, c->neq, kf, row);
     WX_LAUNCHED();
-    WX_CUDA(copy_fortran_plane(c, nbmax, ns, kf, U, false));
+    WX_CUDA(copy_fortran_plane(c, nbmax, ns, kf, U, false, how, row));
   }
   WX_CUDA(cudaStreamSynchronize(c->stream));
   return WX_OK;

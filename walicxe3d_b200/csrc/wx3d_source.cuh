@@ -353,20 +353,22 @@ __global__ void prims_kernel(const double* __restrict__ u, double* __restrict__ 
 }
 
 // The physical cells of one plane (k = kf) of the Fortran array U(nbMax, neq,
-// -1:18, -1:18, -1:18), staged as [j][i][eq][nbmax], <-> native
-// [slot][eq][k][j][i].  The host link bounds these transfers: sending the
+// -1:18, -1:18, -1:18), staged as [j][i][eq][nbmax] with `row` cells per row,
+// <-> native [slot][eq][k][j][i].  The host link bounds these transfers: the
 // physical cells alone (64 % of a plane with its ghosts, and no upload of what
-// a download keeps) took an upload, eight steps and a download of 300 entries
-// of five equations from 6.85 to 4.11 ms (pinned).  A CTA turns 16 x 16 tiles (slots x cells of a row) through
-// shared memory, so both sides move whole 128-byte lines.
+// a download keeps) took 300 entries of five equations up in 1.20 ms instead
+// of 1.64 and down in 1.11 instead of 3.14 (pinned; pageable 2.9 for 5.5 and
+// 3.2 for 11.8).  A CTA turns 16 x 16 tiles (slots x cells of a row) through
+// shared memory, so the native side moves whole 128-byte lines, the slab side
+// too where nbmax is a multiple of 16.
 __device__ __forceinline__ void fortran_tile(double* __restrict__ slab, double* __restrict__ u, int nbmax, int nslots,
-                                             int neq, int kf, bool to_native) {
+                                             int neq, int kf, int row, bool to_native) {
   __shared__ double tile[NC][NC + 1];
   const int a = threadIdx.x & (NC - 1), b = threadIdx.x >> 4;
   const int groups = (nslots + NC - 1) / NC;
   for (int w = blockIdx.x; w < groups * neq * NC; w += gridDim.x) {
     const int j = w % NC, e = (w / NC) % neq, n0 = w / (NC * neq) * NC;
-    double* s = slab + (size_t)nbmax * (e + (size_t)neq * NC * j) + n0;   // + slot + nbmax neq i
+    double* s = slab + (size_t)nbmax * (e + (size_t)neq * row * j) + n0;   // + slot + nbmax neq i
     double* g = u + cell_off(n0, neq, e, 1, j + 1, kf);                   // + i + neq BCELLS slot
     const size_t si = (size_t)nbmax * neq, gs = (size_t)neq * BCELLS;
     if (to_native) {
@@ -384,12 +386,14 @@ __device__ __forceinline__ void fortran_tile(double* __restrict__ slab, double* 
   }
 }
 
-__global__ void __launch_bounds__(256) fortran_to_native(double* slab, double* u, int nbmax, int nslots, int neq, int kf) {
-  fortran_tile(slab, u, nbmax, nslots, neq, kf, true);
+__global__ void __launch_bounds__(256) fortran_to_native(double* slab, double* u, int nbmax, int nslots, int neq, int kf,
+                                                          int row) {
+  fortran_tile(slab, u, nbmax, nslots, neq, kf, row, true);
 }
 
-__global__ void __launch_bounds__(256) native_to_fortran(double* u, double* slab, int nbmax, int nslots, int neq, int kf) {
-  fortran_tile(slab, u, nbmax, nslots, neq, kf, false);
+__global__ void __launch_bounds__(256) native_to_fortran(double* u, double* slab, int nbmax, int nslots, int neq, int kf,
+                                                          int row) {
+  fortran_tile(slab, u, nbmax, nslots, neq, kf, row, false);
 }
 
 // writeBin / warmstart (output.f90:156-213, init.f90:527-623) store each
