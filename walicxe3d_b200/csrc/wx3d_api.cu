@@ -2088,6 +2088,13 @@ int wx3d_run(wx_ctx* c, int32_t nsteps, wx_state* out) {
   return WX_OK;
 }
 
+// The last part of a table of n rows laid out for find_coef: the slope above
+// each row, and the rows per unit of the first column.
+static void append_slopes(std::vector<double>& h, int n) {
+  for (int i = 0; i + 1 < n; ++i) h[2 * (size_t)n + i] = (h[n + i + 1] - h[n + i]) / (h[i + 1] - h[i]);
+  h[3 * (size_t)n] = (n - 1) / (h[n - 1] - h[0]);
+}
+
 int wx3d_set_cooltable(wx_ctx* c, int32_t npts, const double* logT, const double* b) {
   if (!c || !logT || !b) return WX_ERR_INVALID_ARG;
   if (npts < 2) return fail(c, WX_ERR_COOLING_LOAD_COEFS, "cooling table needs at least two rows");
@@ -2097,9 +2104,7 @@ int wx3d_set_cooltable(wx_ctx* c, int32_t npts, const double* logT, const double
     h[i] = logT[i];
     h[npts + i] = -b[i];  // cooltable(2,i) = -b (cooling.f90:163)
   }
-  // the slope above each row and the rows per dex (find_coef)
-  for (int i = 0; i + 1 < npts; ++i) h[2 * (size_t)npts + i] = (h[npts + i + 1] - h[npts + i]) / (h[i + 1] - h[i]);
-  h[3 * (size_t)npts] = (npts - 1) / (h[npts - 1] - h[0]);
+  append_slopes(h, npts);
   cudaFree(c->dCool);
   c->dCool = nullptr;
   WX_CUDA(cudaMalloc(&c->dCool, h.size() * 8));
@@ -2138,11 +2143,12 @@ int wx3d_set_cooltable_metal(wx_ctx* c, int32_t nptsT, int32_t nptsZ, const doub
 int wx3d_set_cooltable_schure(wx_ctx* c, const double* data, int32_t dmc_f) {
   if (!c || !data) return WX_ERR_INVALID_ARG;
   if (dmc_f < 1 || dmc_f > 4) return fail(c, WX_ERR_COOLING_LOAD_COEFS, "dmc_f selects column 2..5 (1..4)");
-  std::vector<double> h(360);
+  std::vector<double> h(3 * 180 + 1);   // laid out as the plain table, for a COOL_TABLE context that loads this one
   for (int i = 0; i < 180; ++i) {
     h[i] = std::pow(10.0, data[5 * i]);
     h[180 + i] = std::pow(10.0, -data[5 * i + dmc_f]);
   }
+  append_slopes(h, 180);
   cudaFree(c->dCool);
   c->dCool = nullptr;
   WX_CUDA(cudaMalloc(&c->dCool, h.size() * 8));
