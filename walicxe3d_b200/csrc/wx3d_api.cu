@@ -537,8 +537,9 @@ int launch_stage(wx_ctx* c, int order, const double* src, const double* base, do
   return WX_OK;
 }
 
-// One CTA per block; where that leaves SMs without their three CTAs, a
-// cluster of up to eight CTAs splits each block's planes.
+// One CTA per block; with fewer than three per SM, what the kernel holds up to
+// six equations (two at seven and eight), a cluster of up to eight CTAs splits
+// each block's planes.
 cudaError_t launch_viscous(const Kern& k, ViscParams V, int nwork, int nsm, cudaStream_t s) {
   V.zsplit = 1;
   while (V.zsplit < 8 && nwork * V.zsplit < 3 * nsm) V.zsplit *= 2;

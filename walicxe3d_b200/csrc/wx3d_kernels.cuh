@@ -111,19 +111,6 @@ __device__ __forceinline__ void block_min_dt(double v, DevCtl* ctl) {
   if ((threadIdx.x & 31) == 0) atomic_min_pos(&ctl->dtmin_bits, v);
 }
 
-// Block-wide sum of four status counters into ctl->cnt.
-__device__ __forceinline__ void flush_counts(DevCtl* ctl, unsigned pf, unsigned df, unsigned zd) {
-  unsigned m = __activemask();
-  pf = __reduce_add_sync(m, pf);
-  df = __reduce_add_sync(m, df);
-  zd = __reduce_add_sync(m, zd);
-  if ((threadIdx.x & 31) == 0) {
-    if (pf) atomicAdd(&ctl->cnt[0], (unsigned long long)pf);
-    if (df) atomicAdd(&ctl->cnt[1], (unsigned long long)df);
-    if (zd) atomicAdd(&ctl->cnt[2], (unsigned long long)zd);
-  }
-}
-
 // One interface flux in direction DIR from ring cells c0..c3 (pointers to
 // equation 0 of cells l-1, l, r, r+1; stride Geo<ORDER>::PL between channels).
 // With CARRY (the z-interfaces, which a thread visits in order along its
@@ -528,7 +515,8 @@ __global__ void __launch_bounds__(STAGE_THREADS, 1) stage_kernel(StageParams P) 
 // same two barriers.  Conserved cells arrive by 8-byte asynchronous copies a
 // plane ahead and stay in shared memory until they are the base of the
 // update (P.base is P.src), so no load holds registers across the fluxes:
-// with 96 registers and no spills two CTAs share an SM.  Loading them into
+// with 96 registers two CTAs share an SM (no spills up to six equations, 12 to
+// 40 bytes of stores at seven).  Loading them into
 // registers instead, or late, spilled or exposed the loads (1.71 and 1.95 ms
 // against 1.51 on the 11,600-block AMR blast at five equations; the kernel
 // that staged everything took 1.75); three CTAs at 64 registers: 2.06 ms.
@@ -776,19 +764,22 @@ __global__ void __launch_bounds__(STAGE_THREADS, 2) predictor_kernel(StageParams
 
 // ---------------------------------------------------------------------------
 // Second-order stage of the hydro equations (the corrector), laid out as the
-// predictor above: columns in registers, block-face interfaces on warps 8
-// and 9, one barrier per plane.  Shared memory holds two planes of
-// primitives with their one-deep x/y frame.  A column thread
+// predictor above: columns on 256 threads, block-face interfaces on warps 8
+// and 9, one barrier per plane.  Shared memory holds a ring of three planes
+// with their one-deep x/y frame: primitives of planes m and m+1, and plane
+// m+2, which arrives as conserved variables.  A column thread
 //  - limits its own x-slope and passes the state at its left face to the
 //    lane below by a shuffle, so every x-slope is computed once;
 //  - limits its own and the next row's y-slope;
-//  - limits the z-slope of the cell above, whose upper-face state it carries
-//    to the next plane's interface; the cell two planes up stays in
-//    registers until it is needed as a plane;
-//  - takes its next source and base cells by asynchronous copies.
-// A face thread keeps both ghost layers of its (side, row) in registers,
-// leaves the inner one in the frame for the slopes next to the face, and
-// solves the block-face interface.
+//  - converts its cell of plane m+2 in place, limits the z-slope of the cell
+//    above, and carries that cell's upper-face state to the next plane's
+//    interface;
+//  - copies its cell of plane m+3 over plane m asynchronously once the
+//    barrier has passed, and loads its base cell, whose plane was brought
+//    into L2 a plane ahead.
+// A face thread leaves the inner ghost of its (side, row) in the frame for the
+// slopes next to the face, keeps the outer one in registers, and solves the
+// block-face interface.
 //
 // VISC (whole blocks) fuses doViscousStep (hydro_solver.f90:217-250): the
 // result W of plane m goes to one of two shared planes framed by the
@@ -798,13 +789,17 @@ __global__ void __launch_bounds__(STAGE_THREADS, 2) predictor_kernel(StageParams
 // same thread) and W(m).
 //
 // Bound, as the predictor, by the shared-memory data path (60 % busy) and
-// instruction issue (50 %) at ten warps per scheduler pair; two CTAs per SM
-// up to six equations need both 96 registers without spills (a plane is
-// converted in place at its z-interface instead of waiting in registers) and
-// at most 113 KB: at six equations the frame rows are unpadded for that.
-// 11,600-block AMR blast, five equations: fused 3.44 -> 2.87 ms, unfused
-// 2.72 -> 2.51 ms; 5,496-block winds mesh, six equations: fused (one CTA per
-// SM before) 2.37 -> 1.90 ms, unfused 1.55 -> 1.36 ms.  The prefetch of the
+// instruction issue (50 %) at five warps per scheduler.  Up to six equations
+// two CTAs share an SM: 96 registers, which the conversion in place keeps
+// almost free of spills (minmod at five equations none, the fused form at six
+// 48 bytes of stores and 124 of loads), and at most 113 KB, for which the
+// frame rows are unpadded.  At seven the unfused form still pairs CTAs, with
+// 48 to 124 bytes of spill stores (1,128 blocks, HLLC and minmod, with the
+// predictor and the viscous kernel: 1.11 -> 0.83 ms against the staged kernel
+// at one CTA), and the fused form runs one at 168 registers (0.98 -> 0.81).
+// 11,600-block AMR blast, five equations: fused 3.44 -> 2.83 ms, unfused
+// 2.72 -> 2.45 ms; 5,496-block winds mesh, six equations: fused (one CTA per
+// SM before) 2.37 -> 1.79 ms, unfused 1.55 -> 1.36 ms.  The prefetch of the
 // next base plane is 4 % of it; keeping the base in a shared plane instead
 // cost 15 % (less L1 for the ghost gathers).
 template <int NEQ, bool VISC>
