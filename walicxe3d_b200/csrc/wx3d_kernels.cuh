@@ -235,8 +235,8 @@ __device__ __forceinline__ void load_plane(const StageParams& P, const DevBlock&
 // One CTA per SM (168 registers, 105-200 KB of shared memory): bound by the
 // FP64 chains of HLLD.  Refined reciprocals and roots in place of its nine
 // divisions and seven roots per interface, and minmod compiled in as for
-// hydro: 440 blocks (HLLD) predictor 0.394 -> 0.270 ms, corrector with the
-// viscous step 0.912 -> 0.430 ms; 16 blocks in 8 slabs 29 + 50 -> 20 + 24 us.
+// hydro: 440 blocks (HLLD) predictor 0.394 -> 0.266 ms, corrector with the
+// viscous step 0.912 -> 0.434 ms; 16 blocks in 8 slabs 29 + 50 -> 20 + 24 us.
 
 // Cell-centred electric field E = -v x B of the stage primitives at one ring
 // cell: the field-interpolated E of the field-CD scheme (Toth 2000, J. Comput.
